@@ -232,7 +232,9 @@ int rbffd_weights_compute(rbffd_grid* grid, const rbffd_weight_params* params, c
  * method performs dgetf2's arithmetic (first-maximum partial pivoting,
  * multipliers by division, fused updates in step order) and gives the same
  * weights bit for bit; they differ in where the system lives:
- *   RBFFD_ELIM_AUTO       the autotuner picks per system size (default);
+ *   RBFFD_ELIM_AUTO       (default) one row per thread, panels of 8 steps whose delayed
+ *                         updates run on the FP64 tensor cores; where a system does not fit
+ *                         shared memory in that form, the fastest of those below, timed;
  *   RBFFD_ELIM_UNBLOCKED  shared memory, one pass over the trailing rows per step;
  *   RBFFD_ELIM_BLOCKED    shared memory, panels of 8 steps with register-tiled updates;
  *   RBFFD_ELIM_ROW_MAP    shared memory, rows never swapped (a row map), one barrier per step;

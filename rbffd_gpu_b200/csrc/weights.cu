@@ -31,6 +31,7 @@
 #include <climits>
 #include <cstring>
 #include <map>
+#include <type_traits>
 #include <vector>
 
 #include "ell.cuh"
@@ -51,8 +52,9 @@ constexpr int MAX_CLASSES = 24;  // system sizes in one persistent launch
 // rows_off + nrows), solved `teams` at a time per CTA by teams of `team`
 // threads, each holding its system at row stride lda in `stride` doubles of
 // shared memory; its work units are numbered from unit0.
+// rpt: panel rows per thread (ELIM_ROWS).
 struct WClass {
-    int m, lda, team, teams, stride, blocked, rows_off, nrows, unit0;
+    int m, lda, team, teams, stride, blocked, rows_off, nrows, unit0, rpt;
 };
 
 struct WParams {
@@ -862,8 +864,19 @@ __device__ SysInputs team_inputs(const Team& T, const WParams& P, int r, double*
     S.x0[0] = x0[0];
     S.x0[1] = x0[1];
     S.x0[2] = x0[2];
-    S.lam_i = atan2(x0[1], x0[0]);
-    S.th_i = atan2(x0[2], sqrt(x0[0] * x0[0] + x0[1] * x0[1]));
+    S.angles = false;
+    bool hv = false;
+    for (int c = 0; c < P.K; c++) {
+        S.angles |= P.opbit[c] == RBFFD_LAMBDA || P.opbit[c] == RBFFD_THETA;
+        hv |= P.opbit[c] == RBFFD_HV;
+    }
+    // the centre's angles: for the operators above and the tangent frame (one thread's)
+    S.lam_i = 0.0;
+    S.th_i = 0.0;
+    if (S.angles || (S.deg >= 2 && T.tid == 0)) {
+        S.lam_i = atan2(x0[1], x0[0]);
+        S.th_i = atan2(x0[2], sqrt(x0[0] * x0[0] + x0[1] * x0[1]));
+    }
     if (S.deg >= 2) {
         if (T.tid == 0) {
             fr[0] = -sin(S.lam_i); fr[1] = cos(S.lam_i); fr[2] = 0.0;
@@ -882,9 +895,7 @@ __device__ SysInputs team_inputs(const Team& T, const WParams& P, int r, double*
         if (T.lane() == 0)
             atomicMax(reinterpret_cast<unsigned long long*>(fr + 7), (unsigned long long)__double_as_longlong(s2));
     }
-    S.angles = false;
-    for (int c = 0; c < P.K; c++) S.angles |= P.opbit[c] == RBFFD_LAMBDA || P.opbit[c] == RBFFD_THETA;
-    S.eps_2k = pow(S.eps, 2 * P.hv_k);
+    S.eps_2k = hv ? pow(S.eps, 2 * P.hv_k) : 0.0;
     T.sync();  // frame and distance visible
     S.s = fr[7] > 0.0 ? sqrt(fr[7]) : 1.0;
     return S;
@@ -898,22 +909,34 @@ __device__ __forceinline__ double phi_pair(const double* xs, int i, int j, doubl
     return g_eval(eps2, r2);
 }
 
-// Polynomial border entry: basis function q at node i.
-__device__ __forceinline__ double poly_entry(const SysInputs& S, const double* xs, const double* fr, int q, int i)
+// Node i's row of the polynomial border: put(q, value) for every basis function q.
+template <typename PutF>
+__device__ __forceinline__ void poly_entries(const SysInputs& S, const double* xs, const double* fr, int i, PutF put)
 {
     if (S.deg >= 2) {
         const double* e1 = fr;
         const double* e2 = fr + 3;
-        int pa, pb;
-        tangent_exp(q, pa, pb);
         double dx = xs[3 * i] - S.x0[0], dy = xs[3 * i + 1] - S.x0[1], dz = xs[3 * i + 2] - S.x0[2];
         double u = __ddiv_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, e1[0]), __dmul_rn(dy, e1[1])), __dmul_rn(dz, e1[2])), S.s);
         double w = __ddiv_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, e2[0]), __dmul_rn(dy, e2[1])), __dmul_rn(dz, e2[2])), S.s);
-        return ipow(u, pa) * ipow(w, pb);
+        // u^a w^b by degree t = a + b, a = t .. 0 (the order of tangent_exp), powers by repeated products
+        double pu[5] = {1.0}, pw[5] = {1.0};
+#pragma unroll
+        for (int t = 1; t < 5; t++) {
+            pu[t] = __dmul_rn(pu[t - 1], u);
+            pw[t] = __dmul_rn(pw[t - 1], w);
+        }
+#pragma unroll
+        for (int t = 0; t < 5; t++)
+            if (t <= S.deg)
+#pragma unroll
+                for (int b = 0; b <= t; b++) put(t * (t + 1) / 2 + b, __dmul_rn(pu[t - b], pw[b]));
+        return;
     }
-    int pa, pb, pc;
-    basis_exp(q, pa, pb, pc);
-    return ipow(xs[3 * i], pa) * ipow(xs[3 * i + 1], pb) * ipow(xs[3 * i + 2], pc);
+    if (S.deg >= 0) put(0, 1.0);
+    if (S.deg == 1)
+#pragma unroll
+        for (int c = 0; c < 3; c++) put(1 + c, xs[3 * i + c]);
 }
 
 // The node quantities a right-hand-side entry of node j < n needs: its
@@ -960,53 +983,57 @@ __device__ __forceinline__ double rhs_poly(const WParams& P, const SysInputs& S,
     return v;
 }
 
-// Team assembly of the augmented system [A | B] of stencil r into a (m rows of
-// m + K columns at row stride ld).  xs: scratch for the stencil's coordinates;
-// fr: 8 doubles of scratch (tangent frame, distance).  Returns m.  Ends with a
-// team barrier.
+// Team assembly of the augmented system [A | B] of stencil r into a: m rows of
+// m + K columns, element (i, j) at a[i * ld + j], or column-major at
+// a[j * ld + i] (A is symmetric: only the right-hand sides differ).  xs:
+// scratch for the stencil's coordinates; fr: 8 doubles of scratch (tangent
+// frame, distance).  Returns m.  Ends with a team barrier.
+template <bool COLS>
 __device__ int team_assemble(const Team& T, const WParams& P, int r, double* a, double* xs, double* fr, int& n_out,
                              int ld)
 {
     const SysInputs S = team_inputs(T, P, r, xs, fr);
     const int n = S.n, np = S.np, m = S.m, K = P.K;
     // Phi block: symmetric to the last bit (x_j - x_i squares to the same
-    // r^2), so each pair j <= i is evaluated once and written to both places:
-    // n(n+1)/2 exponentials.
-    for (int e = T.tid; e < n * (n + 1) / 2; e += T.size) {
-        int i = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);  // e = i(i+1)/2 + j, 0 <= j <= i (estimate, corrected below)
-        while (i * (i + 1) / 2 > e) i--;
-        while ((i + 1) * (i + 2) / 2 <= e) i++;
-        const int j = e - i * (i + 1) / 2;
+    // r^2), so each pair j <= i is evaluated once and written to both places.
+    // Rows q and n-1-q of the lower triangle make one run of n + 1 pairs, so a
+    // thread steps through the pairs without divisions.
+    for (int q = 0, t = T.tid;; t += T.size) {
+        while (t > n) {
+            t -= n + 1;
+            q++;
+        }
+        if (2 * q >= n) break;
+        const bool far = t < n - q;  // in row n - 1 - q, else in row q
+        const int i = far ? n - 1 - q : q, j = far ? t : t - (n - q);
+        if (!far && 2 * q == n - 1) continue;  // the middle row of an odd n is its own partner
         const double v = phi_pair(xs, i, j, S.eps2);
         a[j * ld + i] = v;
         a[i * ld + j] = v;
     }
-    // polynomial border and zero block
-    for (int e = T.tid; e < np * n; e += T.size) {
-        int q = e / n, i = e - q * n;
-        const double v = poly_entry(S, xs, fr, q, i);
-        a[(n + q) * ld + i] = v;
-        a[i * ld + (n + q)] = v;
+    auto rhs = [&](int j, int c) -> double& { return COLS ? a[(m + c) * ld + j] : a[j * ld + m + c]; };
+    // polynomial border, and the right-hand sides, one column per operator in
+    // bit order (rbffd.cpp:106-125); a node's kernel value is evaluated once
+    // for all operators
+    for (int i = T.tid; i < n; i += T.size) {
+        poly_entries(S, xs, fr, i, [&](int q, double v) {
+            a[(n + q) * ld + i] = v;
+            a[i * ld + (n + q)] = v;
+        });
+        const double* xj = xs + 3 * i;
+        const NodeTerms t = node_terms(S, xj);
+        for (int c = 0; c < K; c++) rhs(i, c) = rhs_node(P, S, xj, t, c);
     }
     for (int e = T.tid; e < np * np; e += T.size) a[(n + e / np) * ld + n + e % np] = 0.0;
-    // right-hand sides, one column per operator in bit order (rbffd.cpp:106-125);
-    // a node's kernel value is evaluated once for all operators
-    for (int j = T.tid; j < m; j += T.size) {
-        if (j < n) {
-            const double* xj = xs + 3 * j;
-            const NodeTerms t = node_terms(S, xj);
-            for (int c = 0; c < K; c++) a[j * ld + m + c] = rhs_node(P, S, xj, t, c);
-        } else {
-            for (int c = 0; c < K; c++) a[j * ld + m + c] = rhs_poly(P, S, fr, j, c);
-        }
-    }
+    for (int j = n + T.tid; j < m; j += T.size)
+        for (int c = 0; c < K; c++) rhs(j, c) = rhs_poly(P, S, fr, j, c);
     T.sync();
     n_out = n;
     return m;
 }
 
 // The elimination variants a size class can use (same arithmetic, same results).
-enum { ELIM_UNBLOCKED = 0, ELIM_BLOCKED = 1, ELIM_PERM = 2, ELIM_REG = 3 };
+enum { ELIM_UNBLOCKED = 0, ELIM_BLOCKED = 1, ELIM_PERM = 2, ELIM_REG = 3, ELIM_ROWS = 4 };
 
 // One system end to end by one team: assemble, eliminate, back-substitute,
 // store the weights of row r.  a: the team's shared memory,
@@ -1021,7 +1048,7 @@ __device__ void team_solve(const Team& T, const WParams& P, int r, double* a, in
     int* perm = cand_r + 2 * MAX_WARPS;
     const int K = P.K;
     int n;
-    team_assemble(T, P, r, a, xs, fr, n, lda);
+    team_assemble<false>(T, P, r, a, xs, fr, n, lda);
     const int st = mode == ELIM_BLOCKED ? team_eliminate_blocked<8>(T, a, m, K, lda, cand_v, cand_r)
                    : mode == ELIM_PERM  ? team_eliminate_perm(T, a, m, K, lda, cand_v, cand_r, perm)
                                         : team_eliminate(T, a, m, K, lda, cand_v, cand_r, (double*)perm);
@@ -1227,7 +1254,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 16 ? 1 : 2) k_weights_reg(WPara
         if (u >= P.nunits) break;
         const int r = P.rows[Cc.rows_off + u];
         int n;
-        team_assemble(T, P, r, U, xs, fr, n, lda);  // staged in shared memory, then into registers
+        team_assemble<false>(T, P, r, U, xs, fr, n, lda);  // staged in shared memory, then into registers
         double A[R][C];
 #pragma unroll
         for (int q = 0; q < R; q++)
@@ -1264,6 +1291,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 16 ? 1 : 2) k_weights_reg(WPara
         __syncthreads();
     }
 }
+
+#include "weights_rows.cuh"
 
 // One size class in one persistent launch (the classes of a call run as a
 // sequence of such launches, each with the shared memory and the resident
@@ -1311,7 +1340,7 @@ __global__ void __launch_bounds__(512) k_assemble(WParams P, int team_size, doub
     const size_t sz = (size_t)P.m * (P.m + P.K);
     for (int t = blockIdx.x * teams_per_cta + T.id; t < P.nrows; t += gridDim.x * teams_per_cta) {
         int n;
-        team_assemble(T, P, P.rows[t], a, xs, fr, n, P.m + P.K);
+        team_assemble<false>(T, P, P.rows[t], a, xs, fr, n, P.m + P.K);
         for (size_t e = T.tid; e < sz; e += T.size) out[(size_t)t * sz + e] = a[e];
         T.sync();
     }
@@ -1375,7 +1404,7 @@ constexpr int W_CTA = 256;  // threads per CTA of the persistent launch
 
 // A class's team shape: team width (teams per CTA = W_CTA / team) and the elimination.
 struct WShape {
-    int team, blocked;
+    int team, blocked, rpt = 0;
 };
 
 }  // namespace
@@ -1387,6 +1416,27 @@ static int class_lda(int m, int K) { return (m + K) | 1; }
 static size_t class_stride_bytes(int m, int K, int n_pad)
 {
     return (team_bytes_w(m, K, n_pad, class_lda(m, K)) + 127) / 128 * 128;
+}
+
+// The row-per-thread shape of a class, which every size uses unless the caller
+// forces another elimination: one row per thread and one warp per 32 rows,
+// except two rows per thread of one warp at 33 to 48 unknowns.  There a second
+// warp would be mostly idle and cost a CTA barrier per step: 36 against 44 ns
+// per system at m = 37 (three operators, a full device), while at m = 56 and 60
+// two warps take 80 and 82 ns against 91 and 108 ns.  Against the fastest of the
+// other eliminations: 15.6 / 21 ns (m = 21), 36 / 47 (37), 82 / 153 (60),
+// 232 / 432 (90), 432 / 801 (116), 1273 / 2206 (160, one operator).  team = 0
+// where the system does not fit shared memory in this form.
+static WShape rows_shape(int m, int K, int n_pad, int smem_max)
+{
+    WShape s{0, ELIM_ROWS};
+    if (m > MAX_M) return s;
+    const bool two = m > 32 && m <= 48;
+    const int nw = two ? 1 : (m + 31) / 32;
+    if (rows_smem_bytes(m, K, n_pad, nw) > (size_t)smem_max) return s;
+    s.team = 32 * nw;
+    s.rpt = two ? 2 : 1;
+    return s;
 }
 
 // Candidate shapes of a class: teams whose shared memory fits one CTA.
@@ -1471,6 +1521,19 @@ using RegL = RegElim<16, 8, 4>;
 using RegS = RegElim<8, 8, 2>;
 static bool reg_small(int m, int K) { return m <= 64 && m + K <= 64; }
 
+// The row-per-thread kernel of nw warps and rpt rows per thread.
+static void (*rows_kernel(int nw, int rpt))(WParams)
+{
+    if (rpt == 2) return k_weights_rows<1, 2, 12>;
+    switch (nw) {
+    case 1: return k_weights_rows<1, 1, 16>;
+    case 2: return k_weights_rows<2, 1, 8>;
+    case 3: return k_weights_rows<3, 1, 4>;
+    case 4: return k_weights_rows<4, 1, 2>;
+    default: return k_weights_rows<5, 1, 2>;
+    }
+}
+
 // Kernel, threads per CTA and dynamic shared memory of a one-class P's launch.
 struct ClassLaunch {
     void (*kern)(WParams);
@@ -1481,6 +1544,8 @@ struct ClassLaunch {
 static ClassLaunch class_launch(const WParams& P)
 {
     const WClass& C = P.cls[0];
+    if (C.blocked == ELIM_ROWS)
+        return {rows_kernel(C.team / 32, C.rpt), C.team, rows_smem_bytes(C.m, P.K, P.n_pad, C.team / 32)};
     if (C.blocked == ELIM_REG) {
         if (reg_small(C.m, P.K)) return {k_weights_reg<8, 8, 2>, RegS::THREADS, RegS::smem_bytes(C.m, C.lda, P.n_pad)};
         return {k_weights_reg<16, 8, 4>, RegL::THREADS, RegL::smem_bytes(C.m, C.lda, P.n_pad)};
@@ -1529,7 +1594,7 @@ static void enqueue_persistent(const WParams& P, size_t smem, int grid, cudaStre
 static void number_units(WParams& P)
 {
     WClass& C = P.cls[0];
-    C.teams = C.blocked == ELIM_REG ? 1 : W_CTA / C.team;  // register-resident: one system per CTA
+    C.teams = C.blocked == ELIM_REG || C.blocked == ELIM_ROWS ? 1 : W_CTA / C.team;  // one system per CTA
     C.unit0 = 0;
     P.nunits = (C.nrows + C.teams - 1) / C.teams;
 }
@@ -1685,8 +1750,8 @@ extern "C" int rbffd_weights_compute(rbffd_grid* g, const rbffd_weight_params* p
                            : ctx->weights_elim == RBFFD_ELIM_REGISTERS ? ELIM_REG
                                                                       : -1;
         TuneKey key{200 + K, C.m, g->n_pad, forced + 1, 0};
-        WShape best{0, 0};
-        {
+        WShape best = forced < 0 ? rows_shape(C.m, K, g->n_pad, smem_max) : WShape{0, 0};
+        if (best.team == 0) {
             std::lock_guard<std::mutex> lk(ctx->mu);
             auto it = ctx->tuned.find(key);
             if (it != ctx->tuned.end()) best = WShape{it->second.lanes, it->second.block};
@@ -1746,6 +1811,8 @@ extern "C" int rbffd_weights_compute(rbffd_grid* g, const rbffd_weight_params* p
         }
         C.team = best.team;
         C.blocked = best.blocked;
+        C.rpt = best.rpt;
+        if (C.blocked == ELIM_ROWS) C.lda = rows_lda(C.m, K);
     }
     // the whole batch: one persistent launch per class, largest systems first,
     // captured in a CUDA graph and replayed while the parameters stay the same
