@@ -379,7 +379,8 @@ int rbffd_pde_set_time(rbffd_pde* pde, double t);
 int rbffd_pde_get_time(rbffd_pde* pde, double* t);
 
 enum rbffd_advance_flags {
-    RBFFD_ADVANCE_GRAPH = 0x1,   /* capture the steps in a CUDA graph and replay it */
+    RBFFD_ADVANCE_GRAPH = 0x1,   /* capture the steps in a CUDA graph and replay it (where the steps
+                                    do not run device-resident, see rbffd_pde_advance) */
     RBFFD_ADVANCE_UNFUSED = 0x2, /* plain path: one SpMV launch per operator, separate RHS/axpy
                                     launches and a host synchronisation after every step,
                                     the structure of TimeDependentPDE_CL::advanceRK4
@@ -400,7 +401,15 @@ enum rbffd_advance_flags {
  * (src/pdes/time_dependent_pde.cpp:53-73,172-304), nsteps times.
  * scheme must be 2 (TimeDependentPDE::RK4); EULER (0) and MIDPOINT (1) return
  * RBFFD_ERR_UNSUPPORTED, as the reference's GPU class compiles them out and
- * exits on them (TimeDependentPDE_CL::advance, time_dependent_pde_cl.cpp:350-375). */
+ * exits on them (TimeDependentPDE_CL::advance, time_dependent_pde_cl.cpp:350-375).
+ * Without a shape set (rbffd_pde_set_shape, _set_tiled_shape, _set_arithmetic
+ * RBFFD_ARITH_UNFUSED) and without RBFFD_ADVANCE_UNFUSED or _RESIDENT, grids
+ * whose weights fit the SMs' shared memory, at least in part, advance
+ * device-resident: all steps in cooperative launches of one block per SM that
+ * exchange their boundary values through L2, one lane per row in stencil order
+ * (rbffd_pde_get_shape then reports 1 lane, 256 threads: the per-stage shape
+ * with the same bits).  A block that waits in vain for its neighbours ends the
+ * call with RBFFD_ERR_TIMEOUT. */
 int rbffd_pde_advance(rbffd_pde* pde, int scheme, double dt, int nsteps, int flags);
 /* Heat-equation RK4 that allocates no device memory.  No counterpart in the
  * reference: it exists for callers that cannot let a library allocate on the

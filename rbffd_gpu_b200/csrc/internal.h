@@ -59,7 +59,8 @@ struct rbffd_ctx {
     std::map<TuneKey, Shape> tuned;  // autotuner results per problem shape
     int* d_status = nullptr;         // DEV_STATUS_* written by kernels with bounded waits
     int arith = 0;                   // RBFFD_ARITH_*: FP64 arithmetic of rbffd_apply* and of new FP64 PDEs
-    int weights_elim = 0;            // RBFFD_ELIM_*: elimination of the weight solves (0: autotuned)
+    int weights_elim = 0;            // RBFFD_ELIM_*: elimination of the weight solves (0: the default)
+    int* h_wait = nullptr;           // host-mapped DEV_STATUS_* of the device-resident RK4, made on first use
 };
 
 // Read and clear the context's device status; RBFFD_ERR_TIMEOUT if a kernel gave up waiting.
@@ -85,6 +86,7 @@ struct rbffd_grid {
     std::vector<int> h_iperm;      // caller's node index -> internal row
     std::vector<int> h_len;        // stencil lengths, internal order
     std::map<int, struct Halo*> halos;  // per rows-per-block R, built on first use
+    struct Halo* whole = nullptr;       // grid_halo_whole's
     // The cluster-resident RK4 layout (res_C CTAs of res_R rows; rk4.cu): per
     // CTA a halo of at most res_H nodes, each stencil slot's halo position, and
     // each row's push list (consumer CTA << 12 | halo position).  Built on first use.
@@ -135,9 +137,23 @@ struct Halo {
     // only FP32 paths use it.
     unsigned short* d_lidx_s[4] = {};  // sliced ELL: position read at scheduled slot t
     unsigned short* d_slot_s[4] = {};  // original slot of scheduled slot t, SLOT_FREE for padding
+    // Halos of every row of a block whole (grid_halo_whole): the nodes each
+    // block reads from others with their halo positions, and one word per
+    // block that reads this one without being read by it (position max_halo,
+    // which no slot uses): the lists of the device-resident RK4 (rk4_grid.cuh).
+    int* d_rptr = nullptr;             // [nblocks + 1]
+    int* d_rnode = nullptr;
+    unsigned short* d_rpos = nullptr;
+    int max_read = 0;                  // most entries of one block
+    void* d_whole = nullptr;           // the allocation all of a whole halo's arrays are in
+    size_t b_whole = 0;
 };
 constexpr unsigned short SLOT_FREE = 0xFFFF;
 int grid_halo(rbffd_grid* g, int R, const Halo** out);
+// The halo of blocks of exactly R rows (the last may have fewer), without a cap
+// on outliers, positions in node order, and its lists of words read; built on
+// the device (core.cu).
+int grid_halo_whole(rbffd_grid* g, int R, const Halo** out);
 // The halo of R rows per block with its slot schedule for P rows per
 // wavefront (P = 2, 4 or 8).
 int grid_halo_schedule(rbffd_grid* g, int R, int P, const Halo** out);
@@ -182,6 +198,11 @@ struct rbffd_pde {
     double t = 0.0;
     Shape shape;
     bool forced = false;
+    // Device-resident RK4 (rk4_grid.cuh): stage inputs with their stage numbers (two
+    // buffers, by parity), the next stage number, and whether the last advance ran there
+    void* word = nullptr;
+    unsigned word_tag = 1;
+    bool on_grid = false;
     int arith = 0;  // RBFFD_ARITH_*
     cudaGraphExec_t gexec = nullptr;
     double g_dt = 0.0;

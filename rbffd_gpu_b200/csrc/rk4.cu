@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <new>
 #include <type_traits>
 
@@ -368,6 +369,8 @@ static int launch_resident_t(rbffd_pde* P, const ResidentParams<T>& rp, int C, s
     RBFFD_CUDA_TRY(ctx, cudaLaunchKernelEx(&cfg, kern, rp));
     return RBFFD_OK;
 }
+
+#include "rk4_grid.cuh"
 
 // Multiple tracers: state [N][T_tr]; VEC consecutive tracers per lane, loaded
 // as one 16-byte vector; T_tr / VEC lanes per row share the row's weights and
@@ -1479,6 +1482,7 @@ static void pde_free(rbffd_pde* P)
     dev_free(ctx, P->wf, (size_t)P->g->N32 * P->g->n4 * (P->dtype == RBFFD_F64 ? sizeof(double) : sizeof(float)));
     for (int k = 0; k < 3; k++) dev_free(ctx, P->ws[k], (size_t)P->g->N32 * P->g->n4 * sizeof(float));
     dev_free(ctx, P->comp, (size_t)P->g->N * P->T * sizeof(float));
+    dev_free(ctx, P->word, 4 * n);
     delete P;
 }
 
@@ -1804,6 +1808,10 @@ extern "C" int rbffd_pde_get_shape(rbffd_pde* P, int* lanes, int* block)
     if (!P || !lanes || !block) return RBFFD_ERR_INVALID;
     *lanes = P->shape.lanes;
     *block = P->shape.block;
+    if (!P->forced && P->on_grid) {  // device-resident: one lane per row, the bits of this per-stage shape
+        *lanes = 1;
+        *block = 256;
+    }
     return RBFFD_OK;
 }
 
@@ -2031,6 +2039,217 @@ static int advance_resident(rbffd_pde* P, double dt, int nsteps, int flags)
     return RBFFD_OK;
 }
 
+// ---------------------------------------------------------------------------
+// device-resident RK4 (rk4_grid.cuh)
+
+// Steps per launch: bounds the time other streams' work waits behind one.
+constexpr int GRID_STEPS = 2000;
+
+struct GridGeom {
+    const Halo* h = nullptr;
+    int R = 0, cs = 0, vec = 1, ipt = 0, maxt = 0, threads = 0;
+    size_t smem = 0;
+};
+
+template <typename T>
+static size_t grid_smem_any(int K, int cs, const Halo* h, int R, int T_tr)
+{
+    return grid_smem<T>(K, cs, R, h->max_halo, T_tr, h->max_read);
+}
+
+// Whether, and how, a PDE's advance runs device-resident: where it was faster
+// than the per-stage kernels' best shape (us per stage, 200 steps, per-stage
+// then resident).
+//   T = 1: all grids of up to 1280 rows per SM with at least an eighth of their
+//     chunks on chip.  All of them: 1.94, 1.15 (642 nodes, n = 17, FP64 heat),
+//     2.90, 1.52 (4096, 31, three operators), 3.60, 1.93 (40003, 37, FP32),
+//     5.83, 2.99 (40962, 50, FP64).  A part: 13.2, 10.2 (163842, 50, FP64: 5 of
+//     13), 7.2, 5.6 (the same in FP32: 10 of 13), 31.8, 26.0 (163842, 101, FP64:
+//     5 of 26), 27.5, 20.6 (163842, 31, three operators: 1 of 8); with 2 of 20
+//     it lost (45.1, 51.1 at 120000, 80, three operators).
+//   T > 1, an item per tracer while one CTA's 1024 threads cover them: 6.2, 4.6
+//     (10242, 50, T = 7, FP32), 9.6, 7.9 (9000, 50, T = 16, FP64).
+//   T <= 4 beyond that, an item per 16-byte vector of tracers: 12.7, 10.6
+//     (40962, 50, T = 4, three operators); FP32 only with every chunk on chip
+//     (6.4, 5.7 at n = 50; a part: 9.1, 9.6 at n = 101).  More tracers lost
+//     (8.7, 9.6 at 20000, 50, T = 16): too few warps for their gathers.
+static bool grid_geom(rbffd_pde* P, GridGeom* out)
+{
+    rbffd_ctx* ctx = P->ctx;
+    rbffd_grid* g = P->g;
+    const bool f64 = P->dtype == RBFFD_F64;
+    const int K = streamed_operators(P), es = f64 ? 8 : 4;
+    int optin = 0, coop = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device);
+    if (!coop || ctx->sm_count < 1) return false;
+    GridGeom q;
+    q.R = round_up((g->N + ctx->sm_count - 1) / ctx->sm_count, 32);
+    // items of one tracer while a CTA's 1024 threads cover them; else, up to four tracers, items of a vector
+    const int V = f64 ? 2 : 4;
+    const long long single = (long long)q.R * P->T;
+    q.vec = single > 1024 && P->T <= 4 && P->T % V == 0 ? V : 1;
+    const long long items = single / q.vec;
+    if (items > (P->T <= 4 ? 2 * 640 : 1024)) return false;
+    q.ipt = items <= 1024 ? 1 : 2;
+    q.maxt = q.ipt == 2 ? 640 : (items <= 256 ? 256 : (items <= 512 ? 512 : 1024));
+    const int nr = std::min(g->nc, grid_reg_chunks(K, es, q.ipt));  // chunks in registers
+    const size_t room = (size_t)optin - 256, chunk = (size_t)q.R * (4 * K * es + 8);
+    const int least = (q.vec == 4 ? g->nc : (g->nc + 7) / 8) - nr;            // chunks shared memory has to hold
+    if (least > (int)(room / chunk)) return false;                           // before the halo is built
+    if (grid_halo_whole(g, q.R, &q.h) != RBFFD_OK) return false;
+    q.cs = std::min(g->nc - nr, (int)(room / chunk));
+    auto smem = [&](int cs) {
+        return f64 ? grid_smem_any<double>(K, cs, q.h, q.R, P->T) : grid_smem_any<float>(K, cs, q.h, q.R, P->T);
+    };
+    while (q.cs > 0 && smem(q.cs) > room) q.cs--;
+    if (q.cs < least || smem(q.cs) > room) return false;
+    q.smem = smem(q.cs);
+    q.threads = round_up((int)((items + q.ipt - 1) / q.ipt), 32);
+    if (q.maxt == 256)  // enough threads for the words read, too
+        q.threads = std::max(q.threads, std::min(256, round_up(std::max(1, q.h->max_read * P->T), 32)));
+    *out = q;
+    return true;
+}
+
+template <typename T, int KIND, bool HV>
+static cudaError_t launch_grid_t(const GridParams<T>& gp, const GridGeom& q, cudaStream_t s)
+{
+    constexpr int V = std::is_same<T, float>::value ? 4 : 2;
+    void (*kern)(GridParams<T>) = q.vec > 1 ? (q.ipt > 1        ? k_rk4_grid<T, KIND, HV, V, 2, 640>
+                                               : q.maxt == 256  ? k_rk4_grid<T, KIND, HV, V, 1, 256>
+                                               : q.maxt == 512  ? k_rk4_grid<T, KIND, HV, V, 1, 512>
+                                                                : k_rk4_grid<T, KIND, HV, V, 1, 1024>)
+                                            : (q.ipt > 1        ? k_rk4_grid<T, KIND, HV, 1, 2, 640>
+                                               : q.maxt == 256  ? k_rk4_grid<T, KIND, HV, 1, 1, 256>
+                                               : q.maxt == 512  ? k_rk4_grid<T, KIND, HV, 1, 1, 512>
+                                                                : k_rk4_grid<T, KIND, HV, 1, 1, 1024>);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q.smem);
+    void* args[1] = {(void*)&gp};
+    if (e == cudaSuccess)
+        e = cudaLaunchCooperativeKernel((const void*)kern, dim3(q.h->nblocks), dim3(q.threads), args, q.smem, s);
+    return e;
+}
+
+// Launches of this kind wait on their own CTAs, so two of them never share a
+// device: each goes behind the last one, whatever its stream.
+static cudaError_t grid_ordered(int device, cudaStream_t s, const std::function<cudaError_t()>& launch)
+{
+    constexpr int MAX_DEV = 64;
+    static std::mutex mu[MAX_DEV];
+    static cudaEvent_t last[MAX_DEV] = {};
+    if (device < 0 || device >= MAX_DEV) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(mu[device]);
+    cudaError_t e = cudaSuccess;
+    if (!last[device])
+        e = cudaEventCreateWithFlags(&last[device], cudaEventDisableTiming);
+    else
+        e = cudaStreamWaitEvent(s, last[device], 0);
+    if (e == cudaSuccess) e = launch();
+    if (e == cudaSuccess) e = cudaEventRecord(last[device], s);
+    return e;
+}
+
+template <typename T>
+static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const GridGeom& q, cudaStream_t s, int* status)
+{
+    rbffd_grid* g = P->g;
+    GridParams<T> gp = {};
+    const StageParams<T> s0 = make_params<T>(P, 0, dt), s3 = make_params<T>(P, 3, dt);
+    gp.rows = q.h->d_rows;
+    gp.ptr = q.h->d_ptr;
+    gp.nodes = q.h->d_nodes;
+    gp.lidx = q.h->d_lidx;
+    gp.rptr = q.h->d_rptr;
+    gp.rnode = q.h->d_rnode;
+    gp.rpos = q.h->d_rpos;
+    gp.w[0] = s0.w0;
+    gp.w[1] = s0.w1;
+    gp.w[2] = s0.w2;
+    gp.cu = s0.cu;
+    gp.cv = s0.cv;
+    gp.u = s0.u;
+    gp.comp = (float*)P->comp;
+    gp.word[0] = P->word;
+    gp.word[1] = (char*)P->word + 2 * (size_t)g->N * P->T * sizeof(T);
+    gp.status = status;
+    gp.c[0] = gp.c[1] = s0.c;
+    gp.c[2] = make_params<T>(P, 2, dt).c;
+    gp.c[3] = s3.c;
+    gp.kappa = s0.kappa;
+    gp.nc = g->nc;
+    gp.T_tr = P->T;
+    gp.R = q.R;
+    gp.cs = q.cs;
+    gp.H = q.h->max_halo;
+    gp.nr = q.h->max_read;
+    for (int done = 0; done < nsteps;) {
+        gp.nsteps = std::min(GRID_STEPS, nsteps - done);
+        gp.tag = P->word_tag;
+        const cudaError_t e = grid_ordered(P->ctx->device, s, [&]() {
+            if (P->kind == KIND_HEAT || P->fused) return launch_grid_t<T, KIND_HEAT, false>(gp, q, s);
+            if (P->use_hv) return launch_grid_t<T, KIND_ADVECT, true>(gp, q, s);
+            return launch_grid_t<T, KIND_ADVECT, false>(gp, q, s);
+        });
+        if (e != cudaSuccess) {
+            if (done == 0) return e;
+            return cudaErrorUnknown;  // some of the steps ran
+        }
+        P->word_tag += 4u * (unsigned)gp.nsteps;
+        done += gp.nsteps;
+    }
+    return cudaSuccess;
+}
+
+// *ran: the steps were issued here (else the caller's per-stage path runs them).
+static int advance_grid(rbffd_pde* P, double dt, int nsteps, int flags, bool* ran)
+{
+    *ran = false;
+    rbffd_ctx* ctx = P->ctx;
+    GridGeom q;
+    if (!grid_geom(P, &q)) return RBFFD_OK;
+    const size_t bytes = 4 * (size_t)P->g->N * P->T * (P->dtype == RBFFD_F64 ? 8 : 4);
+    cudaStream_t s = ctx->stream;
+    if (!P->word) {
+        if (dev_alloc(ctx, &P->word, bytes) != RBFFD_OK) return RBFFD_OK;
+        if (cudaMemsetAsync(P->word, 0, bytes, s) != cudaSuccess) {
+            cudaGetLastError();
+            dev_free(ctx, P->word, bytes);
+            P->word = nullptr;
+            return RBFFD_OK;
+        }
+        P->bytes += bytes;
+    }
+    if (!ctx->h_wait) {
+        if (cudaHostAlloc((void**)&ctx->h_wait, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->h_wait = nullptr;
+            return RBFFD_OK;
+        }
+        *ctx->h_wait = DEV_STATUS_OK;
+    }
+    int* status = nullptr;
+    RBFFD_CUDA_TRY(ctx, cudaHostGetDevicePointer((void**)&status, ctx->h_wait, 0));
+    const cudaError_t e = P->dtype == RBFFD_F64 ? advance_grid_t<double>(P, dt, nsteps, q, s, status)
+                                                : advance_grid_t<float>(P, dt, nsteps, q, s, status);
+    if (e == cudaErrorUnknown) return cuda_error(ctx, e, "device-resident RK4");
+    if (e != cudaSuccess) {  // nothing ran: the per-stage kernels serve
+        cudaGetLastError();
+        return RBFFD_OK;
+    }
+    *ran = true;
+    P->on_grid = true;
+    P->t += dt * nsteps;
+    if (!(flags & RBFFD_ADVANCE_ASYNC)) {
+        RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+        if (*(volatile int*)ctx->h_wait != DEV_STATUS_OK) {
+            *ctx->h_wait = DEV_STATUS_OK;
+            return set_error(ctx, RBFFD_ERR_TIMEOUT, "device-resident RK4: a block gave up waiting for its neighbours");
+        }
+    }
+    return RBFFD_OK;
+}
+
 extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps, int flags)
 {
     if (!P) return RBFFD_ERR_INVALID;
@@ -2061,6 +2280,12 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
         }
         return RBFFD_OK;
     }
+    if (!P->forced) {
+        bool ran = false;
+        const int rc = advance_grid(P, dt, nsteps, flags, &ran);
+        if (rc || ran) return rc;
+    }
+    P->on_grid = false;
     if (!P->forced && P->shape.block == 0 && P->shape.tile == 0) P->shape = autotune(P);
     Shape sh = P->shape;
     if (sh.tile > 0) {  // the halo must exist before any capture (building it copies to the device)
