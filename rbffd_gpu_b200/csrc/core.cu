@@ -18,6 +18,7 @@
 #include <iterator>
 #include <new>
 #include <thread>
+#include <type_traits>
 
 #include "ell.cuh"
 #include "internal.h"
@@ -346,6 +347,8 @@ extern "C" int rbffd_grid_destroy(rbffd_grid* g)
     resident_free(g);
     for (auto& kv : g->halos) halo_free(g, kv.second);
     if (g->whole) halo_free(g, g->whole);
+    for (int k = 0; k < 3; k++) dev_free(ctx, g->d_field[k], (k < 2 ? 1 : 2) * (size_t)g->N * sizeof(double));
+    dev_free(ctx, g->d_idx_caller, wsz * sizeof(int));
     delete g;
     return RBFFD_OK;
 }
@@ -1156,6 +1159,156 @@ int grid_apply_dev_plain(rbffd_grid* g, int op, int T_tr, const double* u, doubl
     return RBFFD_OK;
 }
 
+// K2 in the caller's node order: one launch for a whole rbffd_apply(_dev) call.
+// idx: the stencils with the caller's node numbers (grid_caller_index); or the
+// grid's own, u reordered to match or, THROUGH, each taken through perm (internal
+// node -> caller's node).  A row's sum is stored at the caller's node.  U: type of u and out (FP64 host fields of an FP32 call are
+// rounded as they are read).  VEC: tracers per lane, one or a 16-byte vector;
+// T_tr / VEC lanes of a row share its weights and indices.  Slots in stencil
+// order, one lane per (row, vector): k_ell_apply's sums with G = 1.
+//
+// Bound by the gathers (L1) and, on small grids, by the latency of the dependent
+// loads index -> value, so four chunks' loads are in flight for single values.
+template <typename T, typename U, int VEC, bool PLAIN, bool THROUGH>
+__global__ void __launch_bounds__(256) k_apply_caller(const int* __restrict__ idx, const T* __restrict__ w,
+                                                      const int* __restrict__ perm, int nc, int N,
+                                                      const U* __restrict__ u, U* __restrict__ out, int T_tr)
+{
+    const int lanes = T_tr / VEC;
+    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long row = gt / lanes;
+    if (row >= N) return;
+    const int i = (int)row, t = (int)(gt - row * lanes) * VEC;
+    const U* const ut = u + t;
+    T acc[VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; v++) acc[v] = T(0);
+#pragma unroll(VEC == 1 ? 4 : 2)
+    for (int c = 0; c < nc; c++) {
+        const size_t o = sell_off(i, c, nc);
+        const int4 j4 = ld_idx4(idx + o);
+        const int j[4] = {j4.x, j4.y, j4.z, j4.w};
+        T wv[4];
+        ld_w4(w + o, wv);
+        U x[4][VEC];
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            const U* const q = ut + (size_t)(THROUGH ? __ldg(perm + j[s]) : j[s]) * T_tr;
+            if constexpr (VEC == 1) {
+                x[s][0] = __ldg(q);
+            } else if constexpr (sizeof(U) == 4) {
+                const float4 z = __ldg(reinterpret_cast<const float4*>(q));
+                memcpy(x[s], &z, sizeof z);
+            } else {
+                const double2 z = __ldg(reinterpret_cast<const double2*>(q));
+                memcpy(x[s], &z, sizeof z);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+#pragma unroll
+            for (int v = 0; v < VEC; v++) acc[v] = madd<T, PLAIN>(wv[s], (T)x[s][v], acc[v]);
+    }
+    U* const q = out + (size_t)perm[i] * T_tr + t;
+#pragma unroll
+    for (int v = 0; v < VEC; v++) q[v] = (U)acc[v];
+}
+
+// Threads per block: 256, fewer while that leaves SMs without a block.
+static int apply_block(const rbffd_ctx* ctx, long long threads)
+{
+    const long long per_sm = threads / std::max(1, ctx->sm_count);
+    return (int)std::min<long long>(256, std::max<long long>(32, per_sm / 32 * 32));
+}
+
+__global__ void k_caller_index(const int4* __restrict__ idx, const int* __restrict__ perm, size_t n, int4* __restrict__ out)
+{
+    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n) return;
+    const int4 j = idx[e];
+    out[e] = make_int4(perm[j.x], perm[j.y], perm[j.z], perm[j.w]);
+}
+
+// The stencils with the caller's node numbers, made at a grid's 16th application
+// to wide records: a look-up through perm per slot instead takes 137 against 108
+// us a call at N = 163842, n = 101 with 16 FP32 tracers, the allocation 1.7 ms.
+// nullptr before that, and if there is no memory for them.
+static const int* grid_caller_index(rbffd_grid* g)
+{
+    if (g->d_idx_caller || ++g->wide_applies < 16) return g->d_idx_caller;
+    const size_t n = (size_t)g->N32 * g->n4;
+    if (dev_alloc(g->ctx, (void**)&g->d_idx_caller, n * sizeof(int)) != RBFFD_OK) {
+        g->wide_applies = 0;  // asked for again later
+        return nullptr;
+    }
+    g->bytes += n * sizeof(int);
+    k_caller_index<<<(unsigned)((n / 4 + 255) / 256), 256, 0, g->ctx->stream>>>((const int4*)g->d_idx, g->d_perm, n / 4,
+                                                                               (int4*)g->d_idx_caller);
+    return g->d_idx_caller;
+}
+
+template <typename T, typename U, bool PLAIN, bool THROUGH>
+static void launch_apply_caller_t(rbffd_grid* g, const int* idx, const T* w, const U* u, U* out, int T_tr, cudaStream_t s)
+{
+    constexpr int V = 16 / (int)sizeof(U);
+    const bool vec = T_tr % V == 0 && (((uintptr_t)u | (uintptr_t)out) & 15) == 0;
+    const long long threads = (long long)g->N * (vec ? T_tr / V : T_tr);
+    const int B = apply_block(g->ctx, threads);
+    const unsigned nb = (unsigned)((threads + B - 1) / B);
+    if (vec)
+        k_apply_caller<T, U, V, PLAIN, THROUGH><<<nb, B, 0, s>>>(idx, w, g->d_perm, g->nc, g->N, u, out, T_tr);
+    else
+        k_apply_caller<T, U, 1, PLAIN, THROUGH><<<nb, B, 0, s>>>(idx, w, g->d_perm, g->nc, g->N, u, out, T_tr);
+}
+
+// Fields of N doubles kept with the grid: 0 and 1 rbffd_apply's field and
+// derivative, 2 a reordered field (2 N; separate, so that the first calls on
+// grids up to 65536 nodes stay with small allocations); nullptr without memory.
+static double* grid_field(rbffd_grid* g, int k)
+{
+    const size_t bytes = (k < 2 ? 1 : 2) * (size_t)g->N * sizeof(double);
+    if (!g->d_field[k] && dev_alloc(g->ctx, (void**)&g->d_field[k], bytes) == RBFFD_OK) g->bytes += bytes;
+    return g->d_field[k];
+}
+
+// Node records of at most half a 32-byte sector: on grids past 65536 nodes the
+// field is reordered first, since the caller's order spreads a row's neighbours
+// over a sector each, four times the L1 that the internal order takes (35 us
+// against 3 + 17 us at N = 163842, n = 50, FP64, one tracer); below, the numbers
+// go through perm (at N = 40962 10.5 against 2.3 + 7.4 us and a launch more).
+// Wider records are gathered from the caller's order.
+template <typename T, typename U, bool PLAIN>
+static void launch_apply_caller(rbffd_grid* g, const T* w, const U* u, U* out, int T_tr, cudaStream_t s)
+{
+    const int* idx = nullptr;
+    if (T_tr * sizeof(U) > 16) {
+        idx = grid_caller_index(g);
+    } else if (g->N > 65536) {
+        U* const ui = (U*)grid_field(g, 2);
+        if (ui && grid_to_internal(g, u, ui, T_tr, sizeof(U), s) == RBFFD_OK) {
+            idx = g->d_idx;
+            u = ui;
+        }
+    }
+    if (idx)
+        launch_apply_caller_t<T, U, PLAIN, false>(g, idx, w, u, out, T_tr, s);
+    else
+        launch_apply_caller_t<T, U, PLAIN, true>(g, g->d_idx, w, u, out, T_tr, s);
+}
+
+// deriv = the operator's weights on u, device fields in the caller's order, on the context's stream.
+static void apply_caller(rbffd_grid* g, int op, int dtype, int T_tr, const void* u, void* out, bool doubles, cudaStream_t s)
+{
+    if (dtype == RBFFD_F64 && g->ctx->arith == RBFFD_ARITH_UNFUSED)
+        launch_apply_caller<double, double, true>(g, g->d_w64[op], (const double*)u, (double*)out, T_tr, s);
+    else if (dtype == RBFFD_F64)
+        launch_apply_caller<double, double, false>(g, g->d_w64[op], (const double*)u, (double*)out, T_tr, s);
+    else if (doubles)
+        launch_apply_caller<float, double, false>(g, g->d_w32[op], (const double*)u, (double*)out, T_tr, s);
+    else
+        launch_apply_caller<float, float, false>(g, g->d_w32[op], (const float*)u, (float*)out, T_tr, s);
+}
+
 extern "C" int rbffd_ctx_set_arithmetic(rbffd_ctx* ctx, int arith)
 {
     if (!ctx) return RBFFD_ERR_INVALID;
@@ -1172,17 +1325,6 @@ extern "C" int rbffd_ctx_get_arithmetic(rbffd_ctx* ctx, int* arith)
     return RBFFD_OK;
 }
 
-__global__ void k_d2f(const double* __restrict__ a, float* __restrict__ b, int n)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = __double2float_rn(a[i]);
-}
-__global__ void k_f2d(const float* __restrict__ a, double* __restrict__ b, int n)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (double)a[i];
-}
-
 extern "C" int rbffd_apply(rbffd_grid* g, unsigned der_type, int dtype, unsigned start, unsigned count, const double* u,
                            double* deriv)
 {
@@ -1195,42 +1337,21 @@ extern "C" int rbffd_apply(rbffd_grid* g, unsigned der_type, int dtype, unsigned
     rbffd_ctx* ctx = g->ctx;
     cudaSetDevice(ctx->device);
     int N = g->N;
-    size_t b64 = (size_t)N * sizeof(double);
-    double *du = nullptr, *dd = nullptr;
-    float *fu = nullptr, *fd = nullptr;
-    int rc = RBFFD_OK;
-    if ((rc = dev_alloc(ctx, (void**)&du, b64)) || (rc = dev_alloc(ctx, (void**)&dd, b64)) ||
-        (dtype == RBFFD_F32 && ((rc = dev_alloc(ctx, (void**)&fu, N * sizeof(float))) ||
-                                (rc = dev_alloc(ctx, (void**)&fd, N * sizeof(float)))))) {
-        dev_free(ctx, du, b64);
-        dev_free(ctx, dd, b64);
-        dev_free(ctx, fu, N * sizeof(float));
-        return rc;
-    }
+    // the field and its derivative on the device, in the caller's order; kept with the grid
+    const size_t b64 = (size_t)N * sizeof(double);
+    double *const du = grid_field(g, 0), *const dd = grid_field(g, 1);
+    if (!du || !dd) return RBFFD_ERR_OOM;
     cudaStream_t s = ctx->stream;
-    // du: caller order -> dd: internal order -> apply (all rows) -> du -> dd: caller order
+    if (!(dtype == RBFFD_F64 ? (const void*)g->d_w64[op] : (const void*)g->d_w32[op]))
+        return set_error(ctx, RBFFD_ERR_STATE, "weights of operator bit %d not computed", op);
     cudaError_t e = cudaMemcpyAsync(du, u, b64, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) rc = grid_to_internal(g, du, dd, 1, 8, s);
-    if (e == cudaSuccess && rc == RBFFD_OK) {
-        if (dtype == RBFFD_F64) {
-            rc = ctx->arith == RBFFD_ARITH_UNFUSED ? grid_apply_dev_plain(g, op, 1, dd, du, 0, N, s)
-                                                   : grid_apply_dev(g, op, dtype, 1, dd, du, 0, N, 1, s);
-        } else {
-            k_d2f<<<(N + 255) / 256, 256, 0, s>>>(dd, fu, N);
-            rc = grid_apply_dev(g, op, dtype, 1, fu, fd, 0, N, 1, s);
-            if (rc == RBFFD_OK) k_f2d<<<(N + 255) / 256, 256, 0, s>>>(fd, du, N);
-        }
-        if (rc == RBFFD_OK) rc = grid_to_caller(g, du, dd, 1, 8, s);
+    if (e == cudaSuccess) {
+        apply_caller(g, op, dtype, 1, du, dd, true, s);
         e = cudaGetLastError();
     }
-    if (rc == RBFFD_OK && e == cudaSuccess)
+    if (e == cudaSuccess)
         e = cudaMemcpyAsync(deriv + start, dd + start, (size_t)count * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    dev_free(ctx, du, b64);
-    dev_free(ctx, dd, b64);
-    dev_free(ctx, fu, N * sizeof(float));
-    dev_free(ctx, fd, N * sizeof(float));
-    if (rc != RBFFD_OK) return rc;
     if (e != cudaSuccess) return cuda_error(ctx, e, "rbffd_apply");
     return RBFFD_OK;
 }
@@ -1244,25 +1365,27 @@ extern "C" int rbffd_apply_dev(rbffd_grid* g, unsigned der_type, int dtype, int 
     if (op < 0) return set_error(g->ctx, RBFFD_ERR_INVALID, "der_type 0x%x is not a single operator", der_type);
     rbffd_ctx* ctx = g->ctx;
     cudaSetDevice(ctx->device);
-    const int es = dtype == RBFFD_F64 ? 8 : 4;
-    const size_t bytes = (size_t)g->N * ntracers * es;
-    void *tin = nullptr, *tout = nullptr;
-    int rc;
-    if ((rc = dev_alloc(ctx, &tin, bytes)) || (rc = dev_alloc(ctx, &tout, bytes))) {
-        dev_free(ctx, tin, bytes);
-        return rc;
-    }
     cudaStream_t s = ctx->stream;
-    rc = grid_to_internal(g, u_dev, tin, ntracers, es, s);
-    if (rc == RBFFD_OK)
-        rc = dtype == RBFFD_F64 && ctx->arith == RBFFD_ARITH_UNFUSED
-                 ? grid_apply_dev_plain(g, op, ntracers, (const double*)tin, (double*)tout, 0, g->N, s)
-                 : grid_apply_dev(g, op, dtype, ntracers, tin, tout, 0, g->N, 1, s);
-    if (rc == RBFFD_OK) rc = grid_to_caller(g, tout, deriv_dev, ntracers, es, s);
-    cudaError_t e = cudaStreamSynchronize(s);
-    dev_free(ctx, tin, bytes);
-    dev_free(ctx, tout, bytes);
-    if (rc) return rc;
+    if (!(dtype == RBFFD_F64 ? (const void*)g->d_w64[op] : (const void*)g->d_w32[op]))
+        return set_error(ctx, RBFFD_ERR_STATE, "weights of operator bit %d not computed", op);
+    // a result written over the field (or part of it): from a copy
+    const size_t bytes = (size_t)g->N * ntracers * (dtype == RBFFD_F64 ? 8 : 4);
+    void* copy = nullptr;
+    const char *ub = (const char*)u_dev, *db = (const char*)deriv_dev;
+    if (ub < db + bytes && db < ub + bytes) {
+        const int rc = dev_alloc(ctx, &copy, bytes);
+        if (rc) return rc;
+        const cudaError_t e = cudaMemcpyAsync(copy, u_dev, bytes, cudaMemcpyDeviceToDevice, s);
+        if (e != cudaSuccess) {
+            dev_free(ctx, copy, bytes);
+            return cuda_error(ctx, e, "rbffd_apply_dev copy");
+        }
+        u_dev = copy;
+    }
+    apply_caller(g, op, dtype, ntracers, u_dev, deriv_dev, false, s);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    dev_free(ctx, copy, bytes);
     if (e != cudaSuccess) return cuda_error(ctx, e, "rbffd_apply_dev");
     return RBFFD_OK;
 }

@@ -94,6 +94,11 @@ struct rbffd_grid {
     int* d_res_pptr = nullptr;              // [res_C][res_R + 1] push-list ranges
     unsigned short* d_res_pdst = nullptr;   // [res_C][res_P]
     unsigned short* d_res_lidx = nullptr;   // [res_C][n4][res_R]
+    // rbffd_apply*: d_idx in the caller's node numbers (made at the 16th application
+    // to wide records), and fields kept between calls (grid_field, core.cu)
+    int* d_idx_caller = nullptr;
+    int wide_applies = 0;
+    double* d_field[3] = {nullptr, nullptr, nullptr};
     struct WeightsWork* ww = nullptr;   // the weight solver's device workspace and captured launch (weights.cu)
     size_t bytes = 0;
 };
