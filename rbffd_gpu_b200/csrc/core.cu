@@ -156,6 +156,7 @@ extern "C" int rbffd_ctx_destroy(rbffd_ctx* ctx)
     cudaStreamDestroy(ctx->stream);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->h_wait) cudaFreeHost(ctx->h_wait);
+    if (ctx->stage) cudaFree(ctx->stage);
     delete ctx;
     return RBFFD_OK;
 }
@@ -943,25 +944,39 @@ extern "C" int rbffd_grid_nbytes(const rbffd_grid* g, size_t* bytes)
 // ---------------------------------------------------------------------------
 // weights in and out
 
-// host layout [N][n_pad] in the caller's order -> sliced ELL in internal
-// order (internal row i is the caller's row perm[i]), zero beyond the stencil length
+// Rows [c0, c1) of the caller's host layout [N][n_pad] (w_rm: from row c0) <->
+// sliced ELL in internal order (internal row i is the caller's row perm[i]), one
+// thread per row and 4-slot chunk: whole 32-byte sectors on both sides.  Into
+// the grid: zero beyond the stencil length.
 __global__ void k_pad_rows(const double* __restrict__ w_rm, const int* __restrict__ len, const int* __restrict__ perm,
-                           int N, int n_pad, int n4, int nc, double* __restrict__ w)
+                           int N, int n_pad, int nc, int c0, int c1, double* __restrict__ w)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(e / 32 / nc) * 32 + (int)(e % 32), c = (int)(e / 32 % nc);
     if (i >= N) return;
-    int L = len[i];
-    const double* src = w_rm + (size_t)perm[i] * n_pad;
-    for (int s = 0; s < n4; s++) w[sell_elem(i, s, nc)] = (s < L) ? src[s] : 0.0;
+    const int o = perm[i];
+    if (o < c0 || o >= c1) return;
+    const int L = len[i];
+    const double* src = w_rm + (size_t)(o - c0) * n_pad + 4 * c;
+    double* dst = w + sell_off(i, c, nc);
+#pragma unroll
+    for (int s = 0; s < 4; s++) dst[s] = 4 * c + s < L ? src[s] : 0.0;
 }
 
-__global__ void k_unpad_rows(const double* __restrict__ w, const int* __restrict__ perm, int N, int n_pad, int nc,
-                             double* __restrict__ w_rm)
+__global__ void k_unpad_rows(const double* __restrict__ w, const int* __restrict__ perm, int N, int n_pad, int nc, int c0,
+                             int c1, double* __restrict__ w_rm)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(e / 32 / nc) * 32 + (int)(e % 32), c = (int)(e / 32 % nc);
     if (i >= N) return;
-    double* dst = w_rm + (size_t)perm[i] * n_pad;
-    for (int s = 0; s < n_pad; s++) dst[s] = w[sell_elem(i, s, nc)];
+    const int o = perm[i];
+    if (o < c0 || o >= c1) return;
+    double v[4];
+    ld_w4(w + sell_off(i, c, nc), v);
+    double* dst = w_rm + (size_t)(o - c0) * n_pad + 4 * c;
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+        if (4 * c + s < n_pad) dst[s] = v[s];
 }
 
 __global__ void k_cast_f32(const double* __restrict__ a, float* __restrict__ b, size_t n)
@@ -1037,6 +1052,61 @@ int grid_alloc_w64(rbffd_grid* g, int op)
     return RBFFD_OK;
 }
 
+// The context's staging buffer for weights on their way in or out, of the size
+// asked for up to STAGE_MAX (larger moves go in parts), kept until the context
+// ends.  The caller holds ctx->stage_mu and has finished its use of the buffer
+// when it lets go.  An allocation per call took longer than the move itself
+// (0.3 ms at 1 MB).
+constexpr size_t STAGE_MAX = (size_t)16 << 20;
+static int ctx_stage(rbffd_ctx* ctx, size_t want, double** buf, size_t* bytes)
+{
+    want = std::min(want, STAGE_MAX);
+    if (ctx->stage_bytes < want) {
+        dev_free(ctx, ctx->stage, ctx->stage_bytes);
+        ctx->stage = nullptr;
+        ctx->stage_bytes = 0;
+        const int rc = dev_alloc(ctx, (void**)&ctx->stage, want);
+        if (rc) return rc;
+        ctx->stage_bytes = want;
+    }
+    *buf = ctx->stage;
+    *bytes = ctx->stage_bytes;
+    return RBFFD_OK;
+}
+
+// Move one operator's weights between the host layout and w64: in parts of whole rows.
+static int weights_move(rbffd_grid* g, double* w64, const double* in, double* out)
+{
+    rbffd_ctx* ctx = g->ctx;
+    cudaStream_t s = ctx->stream;
+    std::lock_guard<std::mutex> lk(ctx->stage_mu);
+    const size_t row = (size_t)g->n_pad * sizeof(double);
+    double* stage = nullptr;
+    size_t bytes = 0;
+    const int rc = ctx_stage(ctx, (size_t)g->N * row, &stage, &bytes);
+    if (rc) return rc;
+    const int part = (int)std::min<size_t>((size_t)g->N, bytes / row);
+    const unsigned nb = (unsigned)(((size_t)g->N32 * g->nc + 255) / 256);
+    cudaError_t e = cudaSuccess;
+    for (int c0 = 0; e == cudaSuccess && c0 < g->N; c0 += part) {
+        const int c1 = std::min(g->N, c0 + part);
+        const size_t n = (size_t)(c1 - c0) * row;
+        if (in) {
+            e = cudaMemcpyAsync(stage, in + (size_t)c0 * g->n_pad, n, cudaMemcpyHostToDevice, s);
+            if (e != cudaSuccess) break;
+            k_pad_rows<<<nb, 256, 0, s>>>(stage, g->d_len, g->d_perm, g->N, g->n_pad, g->nc, c0, c1, w64);
+            e = cudaGetLastError();
+        } else {
+            k_unpad_rows<<<nb, 256, 0, s>>>(w64, g->d_perm, g->N, g->n_pad, g->nc, c0, c1, stage);
+            e = cudaGetLastError();
+            if (e == cudaSuccess) e = cudaMemcpyAsync(out + (size_t)c0 * g->n_pad, stage, n, cudaMemcpyDeviceToHost, s);
+        }
+    }
+    const cudaError_t f = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = f;
+    return e == cudaSuccess ? RBFFD_OK : cuda_error(ctx, e, in ? "rbffd_weights_set" : "rbffd_weights_get");
+}
+
 extern "C" int rbffd_weights_set(rbffd_grid* g, unsigned der_type, const double* w)
 {
     if (!g || !w) return RBFFD_ERR_INVALID;
@@ -1046,18 +1116,7 @@ extern "C" int rbffd_weights_set(rbffd_grid* g, unsigned der_type, const double*
     cudaSetDevice(ctx->device);
     int rc = grid_alloc_w64(g, op);
     if (rc) return rc;
-    size_t bytes = (size_t)g->N * g->n_pad * sizeof(double);
-    double* tmp = nullptr;
-    if ((rc = dev_alloc(ctx, (void**)&tmp, bytes))) return rc;
-    cudaError_t e = cudaMemcpyAsync(tmp, w, bytes, cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) {
-        k_pad_rows<<<(g->N + 255) / 256, 256, 0, ctx->stream>>>(tmp, g->d_len, g->d_perm, g->N, g->n_pad, g->n4,
-                                                                 g->nc, g->d_w64[op]);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    dev_free(ctx, tmp, bytes);
-    if (e != cudaSuccess) return cuda_error(ctx, e, "rbffd_weights_set");
+    if ((rc = weights_move(g, g->d_w64[op], w, nullptr))) return rc;
     if ((rc = grid_make_f32(g, op))) return rc;
     RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     return RBFFD_OK;
@@ -1069,19 +1128,8 @@ extern "C" int rbffd_weights_get(rbffd_grid* g, unsigned der_type, double* w)
     int op = der_index(der_type);
     if (op < 0) return set_error(g->ctx, RBFFD_ERR_INVALID, "der_type 0x%x is not a single operator", der_type);
     if (!g->d_w64[op]) return set_error(g->ctx, RBFFD_ERR_STATE, "weights for der_type 0x%x not computed", der_type);
-    rbffd_ctx* ctx = g->ctx;
-    cudaSetDevice(ctx->device);
-    size_t bytes = (size_t)g->N * g->n_pad * sizeof(double);
-    double* tmp = nullptr;
-    int rc = dev_alloc(ctx, (void**)&tmp, bytes);
-    if (rc) return rc;
-    k_unpad_rows<<<(g->N + 255) / 256, 256, 0, ctx->stream>>>(g->d_w64[op], g->d_perm, g->N, g->n_pad, g->nc, tmp);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(w, tmp, bytes, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    dev_free(ctx, tmp, bytes);
-    if (e != cudaSuccess) return cuda_error(ctx, e, "rbffd_weights_get");
-    return RBFFD_OK;
+    cudaSetDevice(g->ctx->device);
+    return weights_move(g, g->d_w64[op], nullptr, w);
 }
 
 // ---------------------------------------------------------------------------

@@ -60,6 +60,9 @@ struct rbffd_ctx {
     int* d_status = nullptr;         // DEV_STATUS_* written by kernels with bounded waits
     int arith = 0;                   // RBFFD_ARITH_*: FP64 arithmetic of rbffd_apply* and of new FP64 PDEs
     int weights_elim = 0;            // RBFFD_ELIM_*: elimination of the weight solves (0: the default)
+    double* stage = nullptr;         // weights on their way in or out (core.cu), under stage_mu
+    size_t stage_bytes = 0;
+    std::mutex stage_mu;
     int* h_wait = nullptr;           // host-mapped DEV_STATUS_* of the device-resident RK4, made on first use
 };
 
