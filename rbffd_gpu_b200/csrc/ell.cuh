@@ -45,6 +45,27 @@ __device__ __forceinline__ void ld_w4(const double* p, double (&w)[4])
     w[3] = b.y;
 }
 
+// ld_w4, or (CS) with the lines marked first to be evicted
+template <bool CS>
+__device__ __forceinline__ void ld_w4_stream(const float* p, float (&w)[4])
+{
+    const float4 t = CS ? __ldcs(reinterpret_cast<const float4*>(p)) : __ldg(reinterpret_cast<const float4*>(p));
+    w[0] = t.x;
+    w[1] = t.y;
+    w[2] = t.z;
+    w[3] = t.w;
+}
+template <bool CS>
+__device__ __forceinline__ void ld_w4_stream(const double* p, double (&w)[4])
+{
+    const double2* const q = reinterpret_cast<const double2*>(p);
+    const double2 a = CS ? __ldcs(q) : __ldg(q), b = CS ? __ldcs(q + 1) : __ldg(q + 1);
+    w[0] = a.x;
+    w[1] = a.y;
+    w[2] = b.x;
+    w[3] = b.y;
+}
+
 // four consecutive weights from shared memory (16-byte aligned)
 __device__ __forceinline__ void ld_w4_shared(const float* p, float (&w)[4])
 {

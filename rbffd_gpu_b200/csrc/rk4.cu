@@ -96,6 +96,61 @@ __device__ __forceinline__ void stage_update(const StageParams<T>& p, int i, siz
     }
 }
 
+// stage_update of VEC consecutive values of one row (e the first, 16-byte
+// aligned when VEC > 1): the state arrays move as whole vectors.  Value by value
+// the compiler has to keep each load behind the stores before it, and a warp's
+// 4- or 8-byte accesses lie 16 bytes apart: four (FP32) or two (FP64) times the
+// L1 work.  us per stage, by value and by vector: 11.5, 9.5 (163842 nodes,
+// n = 50, 4 FP32 tracers), 13.9, 12.0 (100000, 50, 8), 38.9, 35.0 (163842, 50, 16).
+template <typename T, int VEC>
+__device__ __forceinline__ void state_load(const T* p, T (&v)[VEC])
+{
+    typedef typename std::conditional<std::is_same<T, float>::value, float4, double2>::type V;
+    static_assert(sizeof(V) == VEC * sizeof(T), "vector width");
+    const V t = *reinterpret_cast<const V*>(p);
+    memcpy(v, &t, sizeof(V));
+}
+template <typename T, int VEC>
+__device__ __forceinline__ void state_store(T* p, const T (&v)[VEC])
+{
+    typedef typename std::conditional<std::is_same<T, float>::value, float4, double2>::type V;
+    V t;
+    memcpy(&t, v, sizeof(V));
+    *reinterpret_cast<V*>(p) = t;
+}
+
+template <typename T, int KIND, bool HV, int VEC>
+__device__ __forceinline__ void stage_update_vec(const StageParams<T>& p, int i, size_t e, const T (&d0)[VEC],
+                                                 const T (&d1)[VEC], const T (&d2)[VEC], T cu, T cv)
+{
+    if constexpr (VEC == 1) {
+        stage_update<T, KIND, HV>(p, i, e, d0[0], d1[0], d2[0], cu, cv);
+    } else {
+        asm volatile("" ::: "memory");  // the state's loads stay behind the gathers, whose registers they would take
+        T u[VEC], acc[VEC] = {}, next[VEC] = {}, comp[VEC] = {};
+        state_load<T, VEC>(p.u + e, u);
+        if (p.stage > 0) state_load<T, VEC>(p.acc + e, acc);
+        const bool cp = std::is_same<T, float>::value && p.comp;
+        if (cp) state_load<T, VEC>(p.comp + e, comp);
+        StageParams<T> q = p;
+#pragma unroll
+        for (int v = 0; v < VEC; v++) {
+            q.u = &u[v];
+            q.acc = &acc[v];
+            q.xnext = &next[v];
+            q.comp = cp ? &comp[v] : nullptr;
+            stage_update<T, KIND, HV>(q, i, 0, d0[v], d1[v], d2[v], cu, cv);
+        }
+        if (p.stage == 3) {
+            state_store<T, VEC>(p.u + e, u);
+            if (cp) state_store<T, VEC>(p.comp + e, comp);
+        } else {
+            state_store<T, VEC>(p.acc + e, acc);
+            state_store<T, VEC>(p.xnext + e, next);
+        }
+    }
+}
+
 // Single tracer, G lanes per row; lane g handles the 4-slot chunks g, g+G, ...
 // With G == 1 the slots are accumulated in stencil order.
 template <typename T, int KIND, bool HV, int G, bool PLAIN = false>
@@ -435,9 +490,7 @@ __global__ void __launch_bounds__(512) k_stage_vec(StageParams<T> p)
         cu = p.cu[i];
         cv = p.cv[i];
     }
-#pragma unroll
-    for (int v = 0; v < VEC; v++)
-        stage_update<T, KIND, HV>(p, i, (size_t)i * p.T_tr + toff + v, d0[v], d1[v], d2[v], cu, cv);
+    stage_update_vec<T, KIND, HV, VEC>(p, i, (size_t)i * p.T_tr + toff, d0, d1, d2, cu, cv);
 }
 
 // Tiled stage kernel: one CTA per block of R consecutive internal rows.  The
@@ -466,7 +519,10 @@ constexpr int TILE_PF_DIST = 2;
 // cost more, so the autotuner decides.
 // NV > 0: the vectors per node (T_tr / VEC) known at compile time, so node
 // offsets in shared memory and state indices are shifts, not multiplies.
-template <typename T, int VEC, int G, int KIND, bool HV, int PF = 0, int NV = 0>
+// CS: the weights' and positions' lines are the first to leave L2 (tile_geom);
+// there three FP32 operators keep the value-by-value update (90 against 106 us
+// at 163842 nodes, n = 101, 16 tracers: the vectors' registers).
+template <typename T, int VEC, int G, int KIND, bool HV, int PF = 0, int NV = 0, bool CS = false>
 __global__ void __launch_bounds__(1024) k_stage_tile(StageParams<T> p, TileParams tp)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -506,13 +562,14 @@ __global__ void __launch_bounds__(1024) k_stage_tile(StageParams<T> p, TileParam
                 }
                 prefetch_l2(tp.lidx + q);
             }
-            const ushort4 l4 = __ldg(reinterpret_cast<const ushort4*>(tp.lidx + o));
+            const ushort4 l4 = CS ? __ldcs(reinterpret_cast<const ushort4*>(tp.lidx + o))
+                                  : __ldg(reinterpret_cast<const ushort4*>(tp.lidx + o));
             const int ll[4] = {l4.x, l4.y, l4.z, l4.w};
             T wa[4], wb[4], wc[4];
-            ld_w4(p.w0 + o, wa);
+            ld_w4_stream<CS>(p.w0 + o, wa);
             if (KIND == KIND_ADVECT) {
-                ld_w4(p.w1 + o, wb);
-                if (HV) ld_w4(p.w2 + o, wc);
+                ld_w4_stream<CS>(p.w1 + o, wb);
+                if (HV) ld_w4_stream<CS>(p.w2 + o, wc);
             }
 #pragma unroll
             for (int k = 0; k < 4; k++) {
@@ -548,9 +605,13 @@ __global__ void __launch_bounds__(1024) k_stage_tile(StageParams<T> p, TileParam
         cu = p.cu[i];
         cv = p.cv[i];
     }
+    const size_t e = (size_t)i * ntr + (size_t)tv * VEC;
+    if constexpr (CS && KIND == KIND_ADVECT && HV && std::is_same<T, float>::value) {
 #pragma unroll
-    for (int v = 0; v < VEC; v++)
-        stage_update<T, KIND, HV>(p, i, (size_t)i * ntr + (size_t)tv * VEC + v, d0[v], d1[v], d2[v], cu, cv);
+        for (int v = 0; v < VEC; v++) stage_update<T, KIND, HV>(p, i, e + v, d0[v], d1[v], d2[v], cu, cv);
+    } else {
+        stage_update_vec<T, KIND, HV, VEC>(p, i, e, d0, d1, d2, cu, cv);
+    }
 }
 
 // Tiled stage kernel with the weight and index stream software-pipelined in
@@ -618,10 +679,7 @@ __global__ void __launch_bounds__(1024) k_stage_tile_pipe(StageParams<T> p, Tile
             }
         }
     }
-#pragma unroll
-    for (int v = 0; v < VEC; v++)
-        stage_update<T, KIND_HEAT, false>(p, i, (size_t)i * ntr + (size_t)tv * VEC + v, d0[v], T(0), T(0), T(0),
-                                          T(0));
+    stage_update_vec<T, KIND_HEAT, false, VEC>(p, i, (size_t)i * ntr + (size_t)tv * VEC, d0, d0, d0, T(0), T(0));
 }
 
 // Asynchronous global -> shared copies of one node record's vector (16, 8 or
@@ -715,10 +773,7 @@ __global__ void __launch_bounds__(1024) k_stage_tile_db(StageParams<T> p, TilePa
                     for (int v = 0; v < VEC; v++) d0[v] = Ar<T>::fma(w[k], xj[v], d0[v]);
                 }
             }
-#pragma unroll
-            for (int v = 0; v < VEC; v++)
-                stage_update<T, KIND_HEAT, false>(p, i, (size_t)i * ntr + (size_t)tv * VEC + v, d0[v], T(0), T(0),
-                                                  T(0), T(0));
+            stage_update_vec<T, KIND_HEAT, false, VEC>(p, i, (size_t)i * ntr + (size_t)tv * VEC, d0, d0, d0, T(0), T(0));
         }
         __syncthreads();  // tile b's buffer is free for the copies issued next iteration
     }
@@ -845,9 +900,7 @@ __global__ void __launch_bounds__(1024) k_stage_tma(StageParams<T> p, TileParams
         cu = p.cu[i];
         cv = p.cv[i];
     }
-#pragma unroll
-    for (int v = 0; v < VEC; v++)
-        stage_update<T, KIND, HV>(p, i, (size_t)i * p.T_tr + (size_t)tv * VEC + v, d0[v], d1[v], d2[v], cu, cv);
+    stage_update_vec<T, KIND, HV, VEC>(p, i, (size_t)i * p.T_tr + (size_t)tv * VEC, d0, d1, d2, cu, cv);
 }
 
 // Unfused right-hand side + stage update from per-operator outputs (the plain path).
@@ -915,6 +968,7 @@ struct TileGeom {
     int pf = 0;      // L2 prefetch of upcoming chunks
     int pipe = 0;    // k_stage_tile_pipe: weights and indices pipelined in registers
     int db = 0;      // k_stage_tile_db: persistent blocks with two halo buffers
+    int cs = 0;      // k_stage_tile: weights and positions marked first to be evicted from L2
     size_t smem = 0;
 };
 
@@ -1027,8 +1081,15 @@ static bool tile_geom(rbffd_pde* P, Shape sh, TileGeom* tg)
         t.stage_bytes = round_up(K * sh.tile * TMA_CS * 4 * es + sh.tile * TMA_CS * 4 * 2, 128);
         t.smem = (size_t)t.halo_bytes + (size_t)TMA_NB * t.stage_bytes + TMA_NB * sizeof(uint64_t);
     }
-    int optin = 0;
+    // A stage that cannot stay in L2 gives up its weights, read once per stage,
+    // before its state, which the next stage reads: us per stage without and
+    // with, 16 FP32 tracers: 75, 69 (163842 nodes, n = 101), 77, 69 (300000, 50),
+    // three operators 101, 90 (163842, 101); one that stays loses (34, 35 at
+    // 163842, 50).
+    int optin = 0, l2 = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, P->ctx->device);
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, P->ctx->device);
+    t.cs = (size_t)P->g->N32 * P->g->n4 * (streamed_operators(P) * es + 2) + 4 * (size_t)P->g->N * P->T * es > (size_t)l2;
     if (t.smem > (size_t)optin) return false;
     *tg = t;
     return true;
@@ -1044,6 +1105,15 @@ static void launch_tile_v(const StageParams<T>& p, const TileParams& tp, const T
         k_stage_tile<T, VEC, 1, KIND, HV, TILE_PF_DIST><<<nb, t.threads, t.smem, s>>>(p, tp);
         return;
     }
+    if constexpr (VEC > 1)
+        if (t.G == 1 && t.cs) {
+            auto kern = t.vpn == 4   ? k_stage_tile<T, VEC, 1, KIND, HV, 0, 4, true>
+                        : t.vpn == 8 ? k_stage_tile<T, VEC, 1, KIND, HV, 0, 8, true>
+                                     : k_stage_tile<T, VEC, 1, KIND, HV, 0, 0, true>;
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem);
+            kern<<<nb, t.threads, t.smem, s>>>(p, tp);
+            return;
+        }
     // one lane per row with the common node widths: compile-time vectors per node
     if (t.G == 1 && (t.vpn == 1 || t.vpn == 4 || t.vpn == 8)) {
         if (t.vpn == 1) {
