@@ -71,6 +71,8 @@ int rbffd_device_count(int* count);
 int rbffd_ctx_create(int device, rbffd_ctx** out);
 int rbffd_ctx_destroy(rbffd_ctx* ctx);
 const char* rbffd_ctx_last_error(const rbffd_ctx* ctx);
+/* Waits for the context's stream.  RBFFD_ERR_TIMEOUT while a PDE of the context
+ * holds a state that an advance left when it gave up waiting (rbffd_pde_advance). */
 int rbffd_ctx_synchronize(rbffd_ctx* ctx);
 /* Bytes this context holds on the device, and the device's free/total bytes. */
 int rbffd_ctx_mem_info(rbffd_ctx* ctx, size_t* held, size_t* free_bytes, size_t* total_bytes);
@@ -408,9 +410,17 @@ enum rbffd_advance_flags {
  * device-resident: all steps in cooperative launches of one block per SM that
  * exchange their boundary values through L2, one lane per row in stencil order
  * (rbffd_pde_get_shape then reports 1 lane, 256 threads: the per-stage shape
- * with the same bits).  A block that waits in vain for its neighbours ends the
- * call with RBFFD_ERR_TIMEOUT. */
+ * with the same bits).  When a block waits in vain for its neighbours, the state
+ * is lost: the call returns RBFFD_ERR_TIMEOUT, or with RBFFD_ADVANCE_ASYNC the
+ * next rbffd_ctx_synchronize, rbffd_pde_get_state or rbffd_pde_advance that finds
+ * it ended does, and these calls on the PDE go on to until rbffd_pde_set_state
+ * gives it a new state.  Steps issued meanwhile do not run, and the PDE's time
+ * returns to that of the last steps known to be complete.  Other PDEs are not
+ * affected. */
 int rbffd_pde_advance(rbffd_pde* pde, int scheme, double dt, int nsteps, int flags);
+/* Polls a block of the device-resident RK4 makes for a neighbour's value before
+ * it gives up (default 2^21, about a second); 0: gives up on any wait. */
+int rbffd_pde_set_poll_limit(rbffd_pde* pde, int polls);
 /* Heat-equation RK4 that allocates no device memory.  No counterpart in the
  * reference: it exists for callers that cannot let a library allocate on the
  * GPU -- applications that reserve the device's memory for their own pool, or

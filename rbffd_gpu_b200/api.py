@@ -637,6 +637,11 @@ class TimeDependentPDE:
         self.ctx.check(self.ctx.L.rbffd_pde_get_time(self.h, ctypes.byref(t)))
         return t.value
 
+    def setPollLimit(self, polls):
+        """Polls a block of the device-resident RK4 makes for a neighbour's value
+        before it gives up (rbffd_pde_set_poll_limit)."""
+        self.ctx.check(self.ctx.L.rbffd_pde_set_poll_limit(self.h, int(polls)), "set_poll_limit")
+
     def setShape(self, lanes_per_row=0, block_threads=0):
         self.ctx.check(self.ctx.L.rbffd_pde_set_shape(self.h, lanes_per_row, block_threads), "set_shape")
 

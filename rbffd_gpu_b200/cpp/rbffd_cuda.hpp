@@ -492,6 +492,8 @@ public:
         return u;
     }
     void setTime(double t) { check(ctx(), rbffd_pde_set_time(h_, t), "setTime"); }
+    // polls of the device-resident RK4 before a wait gives up (rbffd_pde_set_poll_limit)
+    void setPollLimit(int polls) { check(ctx(), rbffd_pde_set_poll_limit(h_, polls), "setPollLimit"); }
     // FP32 PDEs: carry each step's rounding of u + increment into the next (rbffd_pde_set_compensated_state)
     void setCompensatedState(bool on) { check(ctx(), rbffd_pde_set_compensated_state(h_, on ? 1 : 0), "setCompensatedState"); }
     // PDE::checkLocalError (pde.h:120-127): the solution's error norms against

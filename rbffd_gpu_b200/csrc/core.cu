@@ -155,7 +155,7 @@ extern "C" int rbffd_ctx_destroy(rbffd_ctx* ctx)
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
     if (ctx->d_status) cudaFree(ctx->d_status);
-    if (ctx->h_wait) cudaFreeHost(ctx->h_wait);
+    for (int* p : ctx->wait_pages) cudaFreeHost(p);
     if (ctx->stage) cudaFree(ctx->stage);
     delete ctx;
     return RBFFD_OK;
@@ -167,7 +167,41 @@ extern "C" int rbffd_ctx_synchronize(rbffd_ctx* ctx)
 {
     if (!ctx) return RBFFD_ERR_INVALID;
     RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    bool gave_up = false;
+    {
+        std::lock_guard<std::mutex> lk(ctx->mu);
+        for (const int* p : ctx->wait_pages)
+            for (int k = 0; k < WAIT_PAGE; k++) gave_up |= ((const volatile int*)p)[k] != DEV_STATUS_OK;
+    }
+    if (gave_up)
+        return set_error(ctx, RBFFD_ERR_TIMEOUT, "an advance gave up waiting: its PDE's state has to be set again");
     return RBFFD_OK;
+}
+
+int* ctx_wait_slot(rbffd_ctx* ctx)
+{
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    if (ctx->wait_free.empty()) {
+        int* p = nullptr;
+        if (cudaHostAlloc((void**)&p, WAIT_PAGE * sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        memset(p, 0, WAIT_PAGE * sizeof(int));
+        ctx->wait_pages.push_back(p);
+        for (int k = WAIT_PAGE - 1; k >= 0; k--) ctx->wait_free.push_back(p + k);
+    }
+    int* s = ctx->wait_free.back();
+    ctx->wait_free.pop_back();
+    return s;
+}
+
+void ctx_wait_release(rbffd_ctx* ctx, int* slot)
+{
+    if (!slot) return;
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    *(volatile int*)slot = DEV_STATUS_OK;
+    ctx->wait_free.push_back(slot);
 }
 
 extern "C" int rbffd_ctx_mem_info(rbffd_ctx* ctx, size_t* held, size_t* free_bytes, size_t* total_bytes)

@@ -63,8 +63,15 @@ struct rbffd_ctx {
     double* stage = nullptr;         // weights on their way in or out (core.cu), under stage_mu
     size_t stage_bytes = 0;
     std::mutex stage_mu;
-    int* h_wait = nullptr;           // host-mapped DEV_STATUS_* of the device-resident RK4, made on first use
+    // Host-mapped DEV_STATUS_* words of the device-resident RK4, one per PDE
+    // (ctx_wait_slot), in pages of WAIT_PAGE; under mu
+    std::vector<int*> wait_pages, wait_free;
 };
+constexpr int WAIT_PAGE = 1024;
+// A status word for one PDE, DEV_STATUS_OK (nullptr: no memory), and its return
+// once no launch that may write it is left.
+int* ctx_wait_slot(rbffd_ctx* ctx);
+void ctx_wait_release(rbffd_ctx* ctx, int* slot);
 
 // Read and clear the context's device status; RBFFD_ERR_TIMEOUT if a kernel gave up waiting.
 int ctx_check_device_status(rbffd_ctx* ctx);
@@ -211,6 +218,12 @@ struct rbffd_pde {
     void* word = nullptr;
     unsigned word_tag = 1;
     bool on_grid = false;
+    // Its bounded waits: the status word (host-mapped) a launch that gave up leaves
+    // DEV_STATUS_WAIT_TIMEOUT in until the state is set again, the polls a wait
+    // makes, and the time up to which the steps are known to be complete
+    int* wait = nullptr;
+    int poll_limit = 1 << 21;
+    double t_sure = 0.0;
     int arith = 0;  // RBFFD_ARITH_*
     cudaGraphExec_t gexec = nullptr;
     double g_dt = 0.0;

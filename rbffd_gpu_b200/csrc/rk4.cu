@@ -1534,6 +1534,36 @@ size_t pde_bytes(const rbffd_grid* g, const rbffd_pde_params* prm)
     return b;
 }
 
+// The device-resident RK4's stage inputs with their stage numbers, then its gave-up flag.
+static size_t word_bytes(const rbffd_pde* P)
+{
+    return 4 * (size_t)P->g->N * P->T * (P->dtype == RBFFD_F64 ? 8 : 4) + 16;
+}
+static int* word_gave_up(const rbffd_pde* P) { return (int*)((char*)P->word + word_bytes(P) - 16); }
+
+// Whether a device-resident launch that has ended gave up waiting: the state is
+// then a mixture of steps, and the time returns to the last known complete one.
+static bool pde_gave_up(rbffd_pde* P)
+{
+    if (!P->wait || *(volatile int*)P->wait == DEV_STATUS_OK) return false;
+    P->t = P->t_sure;
+    return true;
+}
+static int pde_wait_error(rbffd_pde* P)
+{
+    return set_error(P->ctx, RBFFD_ERR_TIMEOUT,
+                     "device-resident RK4: a block gave up waiting for its neighbours; the state has to be set again");
+}
+
+// Wait for the PDE's stream: its steps are complete then, or lost.
+static int pde_synchronize(rbffd_pde* P)
+{
+    RBFFD_CUDA_TRY(P->ctx, cudaStreamSynchronize(P->ctx->stream));
+    if (pde_gave_up(P)) return pde_wait_error(P);
+    P->t_sure = P->t;
+    return RBFFD_OK;
+}
+
 static void pde_free(rbffd_pde* P)
 {
     if (!P) return;
@@ -1552,7 +1582,8 @@ static void pde_free(rbffd_pde* P)
     dev_free(ctx, P->wf, (size_t)P->g->N32 * P->g->n4 * (P->dtype == RBFFD_F64 ? sizeof(double) : sizeof(float)));
     for (int k = 0; k < 3; k++) dev_free(ctx, P->ws[k], (size_t)P->g->N32 * P->g->n4 * sizeof(float));
     dev_free(ctx, P->comp, (size_t)P->g->N * P->T * sizeof(float));
-    dev_free(ctx, P->word, 4 * n);
+    dev_free(ctx, P->word, word_bytes(P));
+    ctx_wait_release(ctx, P->wait);
     delete P;
 }
 
@@ -1782,6 +1813,12 @@ extern "C" int rbffd_pde_set_state(rbffd_pde* P, const double* u)
         if (P->comp) RBFFD_CUDA_TRY(ctx, cudaMemsetAsync(P->comp, 0, n * sizeof(float), s));
     }
     RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+    if (pde_gave_up(P)) {  // no launch is left: the new state starts afresh
+        RBFFD_CUDA_TRY(ctx, cudaMemsetAsync(word_gave_up(P), 0, sizeof(int), s));
+        RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+        *(volatile int*)P->wait = DEV_STATUS_OK;
+    }
+    P->t_sure = P->t;
     return RBFFD_OK;
 }
 
@@ -1808,21 +1845,28 @@ extern "C" int rbffd_pde_get_state(rbffd_pde* P, double* u)
         RBFFD_CUDA_TRY(ctx, cudaGetLastError());
         RBFFD_CUDA_TRY(ctx, cudaMemcpyAsync(u, P->stage64, n * 8, cudaMemcpyDeviceToHost, s));
     }
-    RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-    return RBFFD_OK;
+    return pde_synchronize(P);
 }
 
 extern "C" int rbffd_pde_set_time(rbffd_pde* P, double t)
 {
     if (!P) return RBFFD_ERR_INVALID;
-    P->t = t;
+    P->t = P->t_sure = t;
     return RBFFD_OK;
 }
 
 extern "C" int rbffd_pde_get_time(rbffd_pde* P, double* t)
 {
     if (!P || !t) return RBFFD_ERR_INVALID;
+    pde_gave_up(P);
     *t = P->t;
+    return RBFFD_OK;
+}
+
+extern "C" int rbffd_pde_set_poll_limit(rbffd_pde* P, int polls)
+{
+    if (!P || polls < 0) return RBFFD_ERR_INVALID;
+    P->poll_limit = polls;
     return RBFFD_OK;
 }
 
@@ -2105,7 +2149,7 @@ static int advance_resident(rbffd_pde* P, double dt, int nsteps, int flags)
                                          : advance_resident_t<float>(P, dt, nsteps, s, false);
     if (rc) return rc;
     P->t += dt * nsteps;
-    if (!(flags & RBFFD_ADVANCE_ASYNC)) RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+    if (!(flags & RBFFD_ADVANCE_ASYNC)) return pde_synchronize(P);
     return RBFFD_OK;
 }
 
@@ -2221,7 +2265,7 @@ static cudaError_t grid_ordered(int device, cudaStream_t s, const std::function<
 }
 
 template <typename T>
-static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const GridGeom& q, cudaStream_t s, int* status)
+static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const GridGeom& q, cudaStream_t s)
 {
     rbffd_grid* g = P->g;
     GridParams<T> gp = {};
@@ -2242,7 +2286,9 @@ static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const Gri
     gp.comp = (float*)P->comp;
     gp.word[0] = P->word;
     gp.word[1] = (char*)P->word + 2 * (size_t)g->N * P->T * sizeof(T);
-    gp.status = status;
+    gp.status = P->wait;  // one address on host and device (unified addressing)
+    gp.gave_up = word_gave_up(P);
+    gp.polls = P->poll_limit;
     gp.c[0] = gp.c[1] = s0.c;
     gp.c[2] = make_params<T>(P, 2, dt).c;
     gp.c[3] = s3.c;
@@ -2278,8 +2324,9 @@ static int advance_grid(rbffd_pde* P, double dt, int nsteps, int flags, bool* ra
     rbffd_ctx* ctx = P->ctx;
     GridGeom q;
     if (!grid_geom(P, &q)) return RBFFD_OK;
-    const size_t bytes = 4 * (size_t)P->g->N * P->T * (P->dtype == RBFFD_F64 ? 8 : 4);
+    const size_t bytes = word_bytes(P);
     cudaStream_t s = ctx->stream;
+    if (!P->wait && !(P->wait = ctx_wait_slot(ctx))) return RBFFD_OK;
     if (!P->word) {
         if (dev_alloc(ctx, &P->word, bytes) != RBFFD_OK) return RBFFD_OK;
         if (cudaMemsetAsync(P->word, 0, bytes, s) != cudaSuccess) {
@@ -2290,18 +2337,8 @@ static int advance_grid(rbffd_pde* P, double dt, int nsteps, int flags, bool* ra
         }
         P->bytes += bytes;
     }
-    if (!ctx->h_wait) {
-        if (cudaHostAlloc((void**)&ctx->h_wait, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
-            cudaGetLastError();
-            ctx->h_wait = nullptr;
-            return RBFFD_OK;
-        }
-        *ctx->h_wait = DEV_STATUS_OK;
-    }
-    int* status = nullptr;
-    RBFFD_CUDA_TRY(ctx, cudaHostGetDevicePointer((void**)&status, ctx->h_wait, 0));
-    const cudaError_t e = P->dtype == RBFFD_F64 ? advance_grid_t<double>(P, dt, nsteps, q, s, status)
-                                                : advance_grid_t<float>(P, dt, nsteps, q, s, status);
+    const cudaError_t e = P->dtype == RBFFD_F64 ? advance_grid_t<double>(P, dt, nsteps, q, s)
+                                                : advance_grid_t<float>(P, dt, nsteps, q, s);
     if (e == cudaErrorUnknown) return cuda_error(ctx, e, "device-resident RK4");
     if (e != cudaSuccess) {  // nothing ran: the per-stage kernels serve
         cudaGetLastError();
@@ -2310,13 +2347,7 @@ static int advance_grid(rbffd_pde* P, double dt, int nsteps, int flags, bool* ra
     *ran = true;
     P->on_grid = true;
     P->t += dt * nsteps;
-    if (!(flags & RBFFD_ADVANCE_ASYNC)) {
-        RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
-        if (*(volatile int*)ctx->h_wait != DEV_STATUS_OK) {
-            *ctx->h_wait = DEV_STATUS_OK;
-            return set_error(ctx, RBFFD_ERR_TIMEOUT, "device-resident RK4: a block gave up waiting for its neighbours");
-        }
-    }
+    if (!(flags & RBFFD_ADVANCE_ASYNC)) return pde_synchronize(P);
     return RBFFD_OK;
 }
 
@@ -2327,6 +2358,7 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
     if (scheme != 2) return set_error(ctx, RBFFD_ERR_UNSUPPORTED, "time scheme %d (only RK4 = 2)", scheme);
     if (nsteps < 0) return set_error(ctx, RBFFD_ERR_INVALID, "nsteps < 0");
     if (nsteps == 0) return RBFFD_OK;
+    if (pde_gave_up(P)) return pde_wait_error(P);
     if (flags & RBFFD_ADVANCE_RESIDENT) return advance_resident(P, dt, nsteps, flags);
     cudaSetDevice(ctx->device);
     cudaStream_t s = ctx->stream;
@@ -2345,8 +2377,9 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
                 int rc = P->dtype == RBFFD_F64 ? unfused_stage<double>(P, st, dt, s) : unfused_stage<float>(P, st, dt, s);
                 if (rc) return rc;
             }
-            RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
             P->t += dt;
+            const int rc = pde_synchronize(P);
+            if (rc) return rc;
         }
         return RBFFD_OK;
     }
@@ -2400,7 +2433,8 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
     RBFFD_CUDA_TRY(ctx, cudaGetLastError());
     P->t += dt * nsteps;
     if (!(flags & RBFFD_ADVANCE_ASYNC)) {
-        RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
+        const int rc = pde_synchronize(P);
+        if (rc) return rc;
         if (sh.tma) return ctx_check_device_status(ctx);
     }
     return RBFFD_OK;

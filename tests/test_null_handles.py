@@ -1,0 +1,6 @@
+"""Null handles and bad arguments of entry points, rejected without a GPU."""
+from rbffd_gpu_b200 import _lib
+
+
+def test_poll_limit():
+    assert _lib.load().rbffd_pde_set_poll_limit(None, 1) == -1
