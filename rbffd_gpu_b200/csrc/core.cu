@@ -153,6 +153,7 @@ extern "C" int rbffd_ctx_destroy(rbffd_ctx* ctx)
     if (!ctx) return RBFFD_ERR_INVALID;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    grid_launches_forget(ctx);
     cudaStreamDestroy(ctx->stream);
     if (ctx->d_status) cudaFree(ctx->d_status);
     for (int* p : ctx->wait_pages) cudaFreeHost(p);

@@ -66,7 +66,12 @@ struct rbffd_ctx {
     // Host-mapped DEV_STATUS_* words of the device-resident RK4, one per PDE
     // (ctx_wait_slot), in pages of WAIT_PAGE; under mu
     std::vector<int*> wait_pages, wait_free;
+    // the last device-resident RK4 launch on the stream, and the most CTAs of
+    // those that may not have ended (grid_ordered, rk4.cu)
+    cudaEvent_t grid_event = nullptr;
+    int grid_blocks = 0;
 };
+void grid_launches_forget(rbffd_ctx* ctx);
 constexpr int WAIT_PAGE = 1024;
 // A status word for one PDE, DEV_STATUS_OK (nullptr: no memory), and its return
 // once no launch that may write it is left.
@@ -217,7 +222,7 @@ struct rbffd_pde {
     // buffers, by parity), the next stage number, and whether the last advance ran there
     void* word = nullptr;
     unsigned word_tag = 1;
-    bool on_grid = false;
+    bool on_grid = false, one_lane = false;  // one_lane: or per stage with its bits
     // Its bounded waits: the status word (host-mapped) a launch that gave up leaves
     // DEV_STATUS_WAIT_TIMEOUT in until the state is set again, the polls a wait
     // makes, and the time up to which the steps are known to be complete

@@ -1922,7 +1922,7 @@ extern "C" int rbffd_pde_get_shape(rbffd_pde* P, int* lanes, int* block)
     if (!P || !lanes || !block) return RBFFD_ERR_INVALID;
     *lanes = P->shape.lanes;
     *block = P->shape.block;
-    if (!P->forced && P->on_grid) {  // device-resident: one lane per row, the bits of this per-stage shape
+    if (!P->forced && P->one_lane) {  // device-resident, or this shape in its place: the same bits
         *lanes = 1;
         *block = 256;
     }
@@ -2156,8 +2156,11 @@ static int advance_resident(rbffd_pde* P, double dt, int nsteps, int flags)
 // ---------------------------------------------------------------------------
 // device-resident RK4 (rk4_grid.cuh)
 
-// Steps per launch: bounds the time other streams' work waits behind one.
+// Steps per launch, at most, and an upper estimate of a launch's time: they bound
+// how long other streams' work waits for the SMs a launch holds.  A launch more
+// costs 4 to 11 us (the weights into shared memory again).
 constexpr int GRID_STEPS = 2000;
+constexpr double GRID_LAUNCH_US = 2e4;
 
 struct GridGeom {
     const Halo* h = nullptr;
@@ -2245,27 +2248,79 @@ static cudaError_t launch_grid_t(const GridParams<T>& gp, const GridGeom& q, cud
     return e;
 }
 
-// Launches of this kind wait on their own CTAs, so two of them never share a
-// device: each goes behind the last one, whatever its stream.
-static cudaError_t grid_ordered(int device, cudaStream_t s, const std::function<cudaError_t()>& launch)
+// Launches of this kind wait on their own CTAs, and a waiting CTA holds its SM.
+// Those that may run at once (one per context, each on its context's stream)
+// therefore never have more CTAs together than the device has SMs: however the
+// CTAs are placed, an SM without any is left for each that is still to start.
+// One that does not fit beside the others' goes behind the largest of them.  Four
+// contexts, 2000 steps of 642 nodes (n = 17, 21 CTAs each): 9.8 ms (39.5 one
+// behind the other, 19.1 with the per-stage kernels).  Two of 40962 (n = 50, 143
+// CTAs), 400 steps: 9.7 ms, one behind the other (13.1 per stage).  Where a grid
+// covers most SMs and leaves them idle in each, the order costs: four of 4096
+// (n = 31, 128 CTAs), 1000 steps: 21.0 ms (14.3 per stage; one alone 5.3 and 8.7).
+struct GridLaunches {
+    std::mutex mu;
+    std::vector<rbffd_ctx*> ctxs;  // contexts that have launched; their grid_event and grid_blocks are under mu
+};
+static GridLaunches* grid_launches(int device)
 {
     constexpr int MAX_DEV = 64;
-    static std::mutex mu[MAX_DEV];
-    static cudaEvent_t last[MAX_DEV] = {};
-    if (device < 0 || device >= MAX_DEV) return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lk(mu[device]);
+    static GridLaunches all[MAX_DEV];
+    return device >= 0 && device < MAX_DEV ? &all[device] : nullptr;
+}
+
+// A context that ends (its stream idle) leaves the list.
+void grid_launches_forget(rbffd_ctx* ctx)
+{
+    GridLaunches* const L = grid_launches(ctx->device);
+    if (!L) return;
+    std::lock_guard<std::mutex> lk(L->mu);
+    L->ctxs.erase(std::remove(L->ctxs.begin(), L->ctxs.end(), ctx), L->ctxs.end());
+    if (ctx->grid_event) cudaEventDestroy(ctx->grid_event);
+    ctx->grid_event = nullptr;
+}
+
+// launch() on the context's stream, `blocks` CTAs.  An error means that nothing was launched.
+static cudaError_t grid_ordered(rbffd_ctx* ctx, int blocks, const std::function<cudaError_t()>& launch)
+{
+    GridLaunches* const L = grid_launches(ctx->device);
+    if (!L) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(L->mu);
     cudaError_t e = cudaSuccess;
-    if (!last[device])
-        e = cudaEventCreateWithFlags(&last[device], cudaEventDisableTiming);
-    else
-        e = cudaStreamWaitEvent(s, last[device], 0);
-    if (e == cudaSuccess) e = launch();
-    if (e == cudaSuccess) e = cudaEventRecord(last[device], s);
-    return e;
+    if (!ctx->grid_event) {
+        e = cudaEventCreateWithFlags(&ctx->grid_event, cudaEventDisableTiming);
+        if (e != cudaSuccess) return e;
+        L->ctxs.push_back(ctx);
+    }
+    std::vector<rbffd_ctx*> busy;  // the others' unfinished launches
+    int total = blocks;
+    for (rbffd_ctx* c : L->ctxs) {
+        if (c->grid_blocks > 0 && cudaEventQuery(c->grid_event) == cudaSuccess) c->grid_blocks = 0;
+        if (c == ctx || c->grid_blocks == 0) continue;
+        busy.push_back(c);
+        total += c->grid_blocks;
+    }
+    cudaGetLastError();  // cudaErrorNotReady
+    std::sort(busy.begin(), busy.end(), [](const rbffd_ctx* a, const rbffd_ctx* b) { return a->grid_blocks > b->grid_blocks; });
+    for (size_t k = 0; k < busy.size() && total > ctx->sm_count; k++) {
+        e = cudaStreamWaitEvent(ctx->stream, busy[k]->grid_event, 0);
+        if (e != cudaSuccess) return e;
+        total -= busy[k]->grid_blocks;
+    }
+    e = launch();
+    if (e != cudaSuccess) return e;
+    if (cudaEventRecord(ctx->grid_event, ctx->stream) == cudaSuccess) {
+        ctx->grid_blocks = std::max(ctx->grid_blocks, blocks);
+    } else {  // the launch cannot be waited for: it ends here
+        cudaGetLastError();
+        cudaStreamSynchronize(ctx->stream);
+        ctx->grid_blocks = 0;
+    }
+    return cudaSuccess;
 }
 
 template <typename T>
-static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const GridGeom& q, cudaStream_t s)
+static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const GridGeom& q, cudaStream_t s, int* done)
 {
     rbffd_grid* g = P->g;
     GridParams<T> gp = {};
@@ -2299,56 +2354,49 @@ static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const Gri
     gp.cs = q.cs;
     gp.H = q.h->max_halo;
     gp.nr = q.h->max_read;
-    for (int done = 0; done < nsteps;) {
-        gp.nsteps = std::min(GRID_STEPS, nsteps - done);
+    // a stage takes at most about 1 us for the exchange and 0.2 ns per multiply-add of a block (the times at grid_geom)
+    const double stage_us = 1.0 + 2e-4 * q.R * g->n4 * streamed_operators(P) * P->T;
+    const int most = (int)std::max(1.0, std::min((double)GRID_STEPS, GRID_LAUNCH_US / (4 * stage_us)));
+    const int launches = (nsteps + most - 1) / most, per = (nsteps + launches - 1) / launches;
+    while (*done < nsteps) {
+        gp.nsteps = std::min(per, nsteps - *done);
         gp.tag = P->word_tag;
-        const cudaError_t e = grid_ordered(P->ctx->device, s, [&]() {
+        const cudaError_t e = grid_ordered(P->ctx, q.h->nblocks, [&]() {
             if (P->kind == KIND_HEAT || P->fused) return launch_grid_t<T, KIND_HEAT, false>(gp, q, s);
             if (P->use_hv) return launch_grid_t<T, KIND_ADVECT, true>(gp, q, s);
             return launch_grid_t<T, KIND_ADVECT, false>(gp, q, s);
         });
-        if (e != cudaSuccess) {
-            if (done == 0) return e;
-            return cudaErrorUnknown;  // some of the steps ran
-        }
+        if (e != cudaSuccess) return e;
         P->word_tag += 4u * (unsigned)gp.nsteps;
-        done += gp.nsteps;
+        *done += gp.nsteps;
     }
     return cudaSuccess;
 }
 
-// *ran: the steps were issued here (else the caller's per-stage path runs them).
-static int advance_grid(rbffd_pde* P, double dt, int nsteps, int flags, bool* ran)
+// Issues steps device-resident; returns how many (the caller's per-stage path runs the rest).
+static int advance_grid(rbffd_pde* P, double dt, int nsteps)
 {
-    *ran = false;
     rbffd_ctx* ctx = P->ctx;
     GridGeom q;
-    if (!grid_geom(P, &q)) return RBFFD_OK;
+    if (!grid_geom(P, &q)) return 0;
     const size_t bytes = word_bytes(P);
     cudaStream_t s = ctx->stream;
-    if (!P->wait && !(P->wait = ctx_wait_slot(ctx))) return RBFFD_OK;
+    if (!P->wait && !(P->wait = ctx_wait_slot(ctx))) return 0;
     if (!P->word) {
-        if (dev_alloc(ctx, &P->word, bytes) != RBFFD_OK) return RBFFD_OK;
+        if (dev_alloc(ctx, &P->word, bytes) != RBFFD_OK) return 0;
         if (cudaMemsetAsync(P->word, 0, bytes, s) != cudaSuccess) {
             cudaGetLastError();
             dev_free(ctx, P->word, bytes);
             P->word = nullptr;
-            return RBFFD_OK;
+            return 0;
         }
         P->bytes += bytes;
     }
-    const cudaError_t e = P->dtype == RBFFD_F64 ? advance_grid_t<double>(P, dt, nsteps, q, s)
-                                                : advance_grid_t<float>(P, dt, nsteps, q, s);
-    if (e == cudaErrorUnknown) return cuda_error(ctx, e, "device-resident RK4");
-    if (e != cudaSuccess) {  // nothing ran: the per-stage kernels serve
-        cudaGetLastError();
-        return RBFFD_OK;
-    }
-    *ran = true;
-    P->on_grid = true;
-    P->t += dt * nsteps;
-    if (!(flags & RBFFD_ADVANCE_ASYNC)) return pde_synchronize(P);
-    return RBFFD_OK;
+    int done = 0;
+    const cudaError_t e = P->dtype == RBFFD_F64 ? advance_grid_t<double>(P, dt, nsteps, q, s, &done)
+                                                : advance_grid_t<float>(P, dt, nsteps, q, s, &done);
+    if (e != cudaSuccess) cudaGetLastError();
+    return done;
 }
 
 extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps, int flags)
@@ -2383,14 +2431,16 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
         }
         return RBFFD_OK;
     }
-    if (!P->forced) {
-        bool ran = false;
-        const int rc = advance_grid(P, dt, nsteps, flags, &ran);
-        if (rc || ran) return rc;
+    const int done = P->forced ? 0 : advance_grid(P, dt, nsteps);
+    P->on_grid = done == nsteps;
+    P->one_lane = done > 0;
+    if (P->on_grid) {
+        P->t += dt * nsteps;
+        return flags & RBFFD_ADVANCE_ASYNC ? RBFFD_OK : pde_synchronize(P);
     }
-    P->on_grid = false;
-    if (!P->forced && P->shape.block == 0 && P->shape.tile == 0) P->shape = autotune(P);
-    Shape sh = P->shape;
+    const int left = nsteps - done;
+    if (!P->forced && !P->one_lane && P->shape.block == 0 && P->shape.tile == 0) P->shape = autotune(P);
+    Shape sh = P->one_lane ? Shape{1, 256} : P->shape;  // the rest of a call with the same bits
     if (sh.tile > 0) {  // the halo must exist before any capture (building it copies to the device)
         const Halo* h = nullptr;
         int rc = grid_halo(P->g, sh.tile, &h);
@@ -2399,7 +2449,7 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
     }
     if (flags & RBFFD_ADVANCE_GRAPH) {
         const int chunk = 25;
-        int full = nsteps / chunk, rest = nsteps % chunk;
+        int full = left / chunk, rest = left % chunk;
         if (full > 0) {
             if (!P->gexec || P->g_dt != dt || P->g_steps != chunk || P->g_shape.lanes != sh.lanes ||
                 P->g_shape.block != sh.block || P->g_shape.tile != sh.tile || P->g_shape.tma != sh.tma ||
@@ -2428,7 +2478,7 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
         }
         run_steps(P, dt, rest, sh);
     } else {
-        run_steps(P, dt, nsteps, sh);
+        run_steps(P, dt, left, sh);
     }
     RBFFD_CUDA_TRY(ctx, cudaGetLastError());
     P->t += dt * nsteps;
