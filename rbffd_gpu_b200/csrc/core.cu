@@ -40,6 +40,17 @@ int set_error(rbffd_ctx* ctx, int status, const char* fmt, ...)
     return status;
 }
 
+KeepError::KeepError(rbffd_ctx* c) : ctx(c)
+{
+    std::lock_guard<std::mutex> lk(ctx->err_mu);
+    msg = ctx->last_error;
+}
+KeepError::~KeepError()
+{
+    std::lock_guard<std::mutex> lk(ctx->err_mu);
+    if (ctx->last_error != msg) ctx->last_error = msg;
+}
+
 int cuda_error(rbffd_ctx* ctx, cudaError_t e, const char* what)
 {
     int st = (e == cudaErrorMemoryAllocation) ? RBFFD_ERR_OOM : RBFFD_ERR_CUDA;
@@ -821,66 +832,93 @@ __global__ void __launch_bounds__(WHOLE_THREADS) k_halo_whole(const int* __restr
     }
 }
 
-int grid_halo_whole(rbffd_grid* g, int R, const Halo** out)
+int grid_halo_whole_sizes(rbffd_grid* g, int R, int* max_halo, int* max_read)
 {
     rbffd_ctx* ctx = g->ctx;
-    if (g->whole && g->whole->R == R) {
-        *out = g->whole;
-        return RBFFD_OK;
-    }
     const int N = g->N, nblocks = (N + R - 1) / R, words = (N + 31) / 32;
     const size_t smem = (size_t)words * 8;
     if (R < 32 || R % 32 || nblocks > WHOLE_MAX_BLOCKS || smem > 160 * 1024)
         return set_error(ctx, RBFFD_ERR_UNSUPPORTED, "whole halos of %d rows for %d nodes", R, N);
-    cudaStream_t s = ctx->stream;
-    int* d_cnt = nullptr;
-    const size_t b_cnt = (size_t)nblocks * (1 + WHOLE_ADJ) * sizeof(int);
-    std::vector<int> cnt((size_t)nblocks * (1 + WHOLE_ADJ));
-    int rc = dev_alloc(ctx, (void**)&d_cnt, b_cnt);
-    if (rc) return rc;
-    cudaError_t e = cudaFuncSetAttribute(k_halo_whole<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_halo_whole<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) {
-        k_halo_whole<false><<<nblocks, WHOLE_THREADS, smem, s>>>(g->d_idx, N, g->nc, R, words, d_cnt,
-                                                                 (unsigned*)(d_cnt + nblocks), nullptr, nullptr, nullptr,
-                                                                 nullptr, 0, nullptr, nullptr, nullptr, nullptr);
-        e = cudaGetLastError();
+    if (g->whole_R != R) {
+        cudaStream_t s = ctx->stream;
+        int* d_cnt = nullptr;
+        const size_t b_cnt = (size_t)nblocks * (1 + WHOLE_ADJ) * sizeof(int);
+        std::vector<int> cnt((size_t)nblocks * (1 + WHOLE_ADJ));
+        const int rc = dev_alloc(ctx, (void**)&d_cnt, b_cnt);
+        if (rc) return rc;
+        cudaError_t e =
+            cudaFuncSetAttribute(k_halo_whole<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) {
+            k_halo_whole<false><<<nblocks, WHOLE_THREADS, smem, s>>>(g->d_idx, N, g->nc, R, words, d_cnt,
+                                                                     (unsigned*)(d_cnt + nblocks), nullptr, nullptr,
+                                                                     nullptr, nullptr, 0, nullptr, nullptr, nullptr,
+                                                                     nullptr);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.data(), d_cnt, b_cnt, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        dev_free(ctx, d_cnt, b_cnt);
+        if (e != cudaSuccess) return cuda_error(ctx, e, "grid_halo_whole");
+        // offsets, and the words that keep a block behind one that reads it without being read by it; uploaded
+        // together: rows, ptr, rptr and eptr (nblocks + 1 each), then the extra words
+        const unsigned* adj = (const unsigned*)(cnt.data() + nblocks);
+        auto reads = [&](int b, int o) { return adj[b * WHOLE_ADJ + (o >> 5)] >> (o & 31) & 1; };
+        const int nb1 = nblocks + 1;
+        std::vector<int> meta(4 * (size_t)nb1, 0);
+        int *const rows = meta.data(), *const ptr = rows + nb1, *const rptr = ptr + nb1, *const eptr = rptr + nb1;
+        std::vector<int> extra;
+        g->whole_max_halo = g->whole_max_read = 0;
+        for (int b = 0; b < nblocks; b++) {
+            rows[b] = b * R;
+            const int nrows = std::min(N, (b + 1) * R) - b * R;
+            for (int o = 0; o < nblocks; o++)
+                if (o != b && reads(o, b) && !reads(b, o)) extra.push_back(o * R);
+            eptr[b + 1] = (int)extra.size();
+            ptr[b + 1] = ptr[b] + cnt[b];
+            const int nread = cnt[b] - nrows + eptr[b + 1] - eptr[b];
+            rptr[b + 1] = rptr[b] + nread;
+            g->whole_max_halo = std::max(g->whole_max_halo, cnt[b]);
+            g->whole_max_read = std::max(g->whole_max_read, nread);
+        }
+        rows[nblocks] = N;
+        meta.insert(meta.end(), extra.begin(), extra.end());
+        g->whole_refused = g->whole_max_halo > 65534;
+        g->whole_meta = g->whole_refused ? std::vector<int>() : std::move(meta);
+        g->whole_R = R;
+        if (g->whole) {  // one block size at a time: the device's SM count fixes it
+            cudaStreamSynchronize(s);
+            g->bytes -= g->whole->b_whole;
+            halo_free(g, g->whole);
+            g->whole = nullptr;
+        }
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.data(), d_cnt, b_cnt, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    dev_free(ctx, d_cnt, b_cnt);
-    if (e != cudaSuccess) return cuda_error(ctx, e, "grid_halo_whole");
-    // offsets, and the words that keep a block behind one that reads it without being read by it; uploaded
-    // together: rows, ptr, rptr and eptr (nblocks + 1 each), then the extra words
-    const unsigned* adj = (const unsigned*)(cnt.data() + nblocks);
-    auto reads = [&](int b, int o) { return adj[b * WHOLE_ADJ + (o >> 5)] >> (o & 31) & 1; };
-    const int nb1 = nblocks + 1;
-    std::vector<int> meta(4 * (size_t)nb1, 0);
-    int *const rows = meta.data(), *const ptr = rows + nb1, *const rptr = ptr + nb1, *const eptr = rptr + nb1;
-    std::vector<int> extra;
+    if (g->whole_refused) return set_error(ctx, RBFFD_ERR_UNSUPPORTED, "a block halo exceeds 65534 nodes");
+    *max_halo = g->whole_max_halo;
+    *max_read = g->whole_max_read;
+    return RBFFD_OK;
+}
+
+int grid_halo_whole(rbffd_grid* g, int R, const Halo** out)
+{
+    rbffd_ctx* ctx = g->ctx;
     int max_halo = 0, max_read = 0;
-    for (int b = 0; b < nblocks; b++) {
-        rows[b] = b * R;
-        const int nrows = std::min(N, (b + 1) * R) - b * R;
-        for (int o = 0; o < nblocks; o++)
-            if (o != b && reads(o, b) && !reads(b, o)) extra.push_back(o * R);
-        eptr[b + 1] = (int)extra.size();
-        ptr[b + 1] = ptr[b] + cnt[b];
-        const int nread = cnt[b] - nrows + eptr[b + 1] - eptr[b];
-        rptr[b + 1] = rptr[b] + nread;
-        max_halo = std::max(max_halo, cnt[b]);
-        max_read = std::max(max_read, nread);
+    int rc = grid_halo_whole_sizes(g, R, &max_halo, &max_read);
+    if (rc) return rc;
+    if (g->whole) {
+        *out = g->whole;
+        return RBFFD_OK;
     }
-    rows[nblocks] = N;
-    if (max_halo > 65534) return set_error(ctx, RBFFD_ERR_UNSUPPORTED, "a block halo exceeds 65534 nodes");
+    const int N = g->N, nblocks = (N + R - 1) / R, words = (N + 31) / 32, nb1 = nblocks + 1;
+    const size_t smem = (size_t)words * 8;
+    cudaStream_t s = ctx->stream;
     Halo* h = new (std::nothrow) Halo();
     if (!h) return RBFFD_ERR_OOM;
     h->R = R;
     h->nblocks = nblocks;
     h->max_halo = max_halo;
     h->max_read = max_read;
-    const size_t nlidx = (size_t)g->N32 * g->n4, nhalo = (size_t)ptr[nblocks], nread = (size_t)rptr[nblocks];
-    meta.insert(meta.end(), extra.begin(), extra.end());
+    const std::vector<int>& meta = g->whole_meta;
+    const size_t nlidx = (size_t)g->N32 * g->n4, nhalo = (size_t)meta[nb1 + nblocks], nread = (size_t)meta[2 * nb1 + nblocks];
     // one allocation: lidx | rpos | rnode | nodes | meta (16-bit arrays of even length first)
     h->b_whole = (round_up((int)nread, 2) + nlidx) * sizeof(unsigned short) +
                  (nread + nhalo + meta.size()) * sizeof(int);
@@ -895,7 +933,9 @@ int grid_halo_whole(rbffd_grid* g, int R, const Halo** out)
     h->d_rows = h->d_nodes + nhalo;
     h->d_ptr = h->d_rows + nb1;
     h->d_rptr = h->d_ptr + nb1;
-    e = cudaMemcpyAsync(h->d_rows, meta.data(), meta.size() * sizeof(int), cudaMemcpyHostToDevice, s);
+    cudaError_t e = cudaFuncSetAttribute(k_halo_whole<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(h->d_rows, meta.data(), meta.size() * sizeof(int), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
         k_halo_whole<true><<<nblocks, WHOLE_THREADS, smem, s>>>(g->d_idx, N, g->nc, R, words, nullptr, nullptr, h->d_ptr,
                                                                 h->d_rptr, h->d_rptr + nb1, h->d_rptr + 2 * nb1, max_halo,
@@ -907,10 +947,7 @@ int grid_halo_whole(rbffd_grid* g, int R, const Halo** out)
         halo_free(g, h);
         return cuda_error(ctx, e, "grid_halo_whole fill");
     }
-    if (g->whole) {  // one block size at a time: the device's SM count fixes it
-        g->bytes -= g->whole->b_whole;
-        halo_free(g, g->whole);
-    }
+    g->whole_meta = std::vector<int>();
     g->whole = h;
     g->bytes += h->b_whole;
     *out = h;

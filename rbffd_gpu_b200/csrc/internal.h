@@ -102,6 +102,11 @@ struct rbffd_grid {
     std::vector<int> h_len;        // stencil lengths, internal order
     std::map<int, struct Halo*> halos;  // per rows-per-block R, built on first use
     struct Halo* whole = nullptr;       // grid_halo_whole's
+    // The sizes of whole halos of whole_R rows (grid_halo_whole_sizes): refused
+    // past 65534 positions; whole_meta: their offsets, until the halo is made
+    int whole_R = 0, whole_max_halo = 0, whole_max_read = 0;
+    bool whole_refused = false;
+    std::vector<int> whole_meta;
     // The cluster-resident RK4 layout (res_C CTAs of res_R rows; rk4.cu): per
     // CTA a halo of at most res_H nodes, each stencil slot's halo position, and
     // each row's push list (consumer CTA << 12 | halo position).  Built on first use.
@@ -174,6 +179,15 @@ int grid_halo(rbffd_grid* g, int R, const Halo** out);
 // on outliers, positions in node order, and its lists of words read; built on
 // the device (core.cu).
 int grid_halo_whole(rbffd_grid* g, int R, const Halo** out);
+// Its most positions and most words read, without making it; counted once per grid and R.
+int grid_halo_whole_sizes(rbffd_grid* g, int R, int* max_halo, int* max_read);
+// Keeps the context's last error message over work whose failure the caller makes up for.
+struct KeepError {
+    rbffd_ctx* ctx;
+    std::string msg;
+    explicit KeepError(rbffd_ctx* c);
+    ~KeepError();
+};
 // The halo of R rows per block with its slot schedule for P rows per
 // wavefront (P = 2, 4 or 8).
 int grid_halo_schedule(rbffd_grid* g, int R, int P, const Halo** out);
@@ -229,6 +243,7 @@ struct rbffd_pde {
     int* wait = nullptr;
     int poll_limit = 1 << 21;
     double t_sure = 0.0;
+    int grid_skip = 0;  // advances left before memory it did not get is asked for again
     int arith = 0;  // RBFFD_ARITH_*
     cudaGraphExec_t gexec = nullptr;
     double g_dt = 0.0;

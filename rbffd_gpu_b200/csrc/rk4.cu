@@ -2168,12 +2168,6 @@ struct GridGeom {
     size_t smem = 0;
 };
 
-template <typename T>
-static size_t grid_smem_any(int K, int cs, const Halo* h, int R, int T_tr)
-{
-    return grid_smem<T>(K, cs, R, h->max_halo, T_tr, h->max_read);
-}
-
 // Whether, and how, a PDE's advance runs device-resident: where it was faster
 // than the per-stage kernels' best shape (us per stage, 200 steps, per-stage
 // then resident).
@@ -2214,17 +2208,18 @@ static bool grid_geom(rbffd_pde* P, GridGeom* out)
     const size_t room = (size_t)optin - 256, chunk = (size_t)q.R * (4 * K * es + 8);
     const int least = (q.vec == 4 ? g->nc : (g->nc + 7) / 8) - nr;            // chunks shared memory has to hold
     if (least > (int)(room / chunk)) return false;                           // before the halo is built
-    if (grid_halo_whole(g, q.R, &q.h) != RBFFD_OK) return false;
+    int H = 0, words = 0;
+    if (grid_halo_whole_sizes(g, q.R, &H, &words) != RBFFD_OK) return false;
     q.cs = std::min(g->nc - nr, (int)(room / chunk));
     auto smem = [&](int cs) {
-        return f64 ? grid_smem_any<double>(K, cs, q.h, q.R, P->T) : grid_smem_any<float>(K, cs, q.h, q.R, P->T);
+        return f64 ? grid_smem<double>(K, cs, q.R, H, P->T, words) : grid_smem<float>(K, cs, q.R, H, P->T, words);
     };
     while (q.cs > 0 && smem(q.cs) > room) q.cs--;
     if (q.cs < least || smem(q.cs) > room) return false;
     q.smem = smem(q.cs);
     q.threads = round_up((int)((items + q.ipt - 1) / q.ipt), 32);
     if (q.maxt == 256)  // enough threads for the words read, too
-        q.threads = std::max(q.threads, std::min(256, round_up(std::max(1, q.h->max_read * P->T), 32)));
+        q.threads = std::max(q.threads, std::min(256, round_up(std::max(1, words * P->T), 32)));
     *out = q;
     return true;
 }
@@ -2377,8 +2372,15 @@ static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const Gri
 static int advance_grid(rbffd_pde* P, double dt, int nsteps)
 {
     rbffd_ctx* ctx = P->ctx;
+    if (P->grid_skip > 0) {
+        P->grid_skip--;
+        return 0;
+    }
+    KeepError keep(ctx);  // the per-stage path serves whatever fails here
     GridGeom q;
     if (!grid_geom(P, &q)) return 0;
+    P->grid_skip = 64;  // until the memory below is there
+    if (grid_halo_whole(P->g, q.R, &q.h) != RBFFD_OK) return 0;
     const size_t bytes = word_bytes(P);
     cudaStream_t s = ctx->stream;
     if (!P->wait && !(P->wait = ctx_wait_slot(ctx))) return 0;
@@ -2392,6 +2394,7 @@ static int advance_grid(rbffd_pde* P, double dt, int nsteps)
         }
         P->bytes += bytes;
     }
+    P->grid_skip = 0;
     int done = 0;
     const cudaError_t e = P->dtype == RBFFD_F64 ? advance_grid_t<double>(P, dt, nsteps, q, s, &done)
                                                 : advance_grid_t<float>(P, dt, nsteps, q, s, &done);
