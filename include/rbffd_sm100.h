@@ -416,7 +416,10 @@ enum rbffd_advance_flags {
  * it ended does, and these calls on the PDE go on to until rbffd_pde_set_state
  * gives it a new state.  Steps issued meanwhile do not run, and the PDE's time
  * returns to that of the last steps known to be complete.  Other PDEs are not
- * affected. */
+ * affected.
+ * While the caller captures the context's stream (rbffd_ctx_stream) in a CUDA
+ * graph, RBFFD_ADVANCE_ASYNC calls record their stage launches, without a shape
+ * set or tuned before with one lane per row. */
 int rbffd_pde_advance(rbffd_pde* pde, int scheme, double dt, int nsteps, int flags);
 /* Polls a block of the device-resident RK4 makes for a neighbour's value before
  * it gives up (default 2^21, about a second); 0: gives up on any wait. */

@@ -2434,9 +2434,14 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
         }
         return RBFFD_OK;
     }
-    const int done = P->forced ? 0 : advance_grid(P, dt, nsteps);
+    // A caller's capture of the stream records the per-stage launches: a
+    // device-resident launch has its stage numbers once, and tuning waits.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    RBFFD_CUDA_TRY(ctx, cudaStreamIsCapturing(s, &cap));
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    const int done = P->forced || capturing ? 0 : advance_grid(P, dt, nsteps);
     P->on_grid = done == nsteps;
-    P->one_lane = done > 0;
+    P->one_lane = done > 0 || (capturing && !P->forced && P->shape.block == 0 && P->shape.tile == 0);
     if (P->on_grid) {
         P->t += dt * nsteps;
         return flags & RBFFD_ADVANCE_ASYNC ? RBFFD_OK : pde_synchronize(P);
@@ -2450,7 +2455,7 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
         if (rc) return rc;
         if (sh.sched && (rc = pde_sched_prepare(P, sh.tile))) return rc;
     }
-    if (flags & RBFFD_ADVANCE_GRAPH) {
+    if ((flags & RBFFD_ADVANCE_GRAPH) && !capturing) {
         const int chunk = 25;
         int full = left / chunk, rest = left % chunk;
         if (full > 0) {
