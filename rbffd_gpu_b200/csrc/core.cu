@@ -1457,6 +1457,7 @@ extern "C" int rbffd_apply(rbffd_grid* g, unsigned der_type, int dtype, unsigned
     rbffd_ctx* ctx = g->ctx;
     cudaSetDevice(ctx->device);
     int N = g->N;
+    std::lock_guard<std::mutex> lk(g->apply_mu);
     // the field and its derivative on the device, in the caller's order; kept with the grid
     const size_t b64 = (size_t)N * sizeof(double);
     double *const du = grid_field(g, 0), *const dd = grid_field(g, 1);
@@ -1488,6 +1489,7 @@ extern "C" int rbffd_apply_dev(rbffd_grid* g, unsigned der_type, int dtype, int 
     cudaStream_t s = ctx->stream;
     if (!(dtype == RBFFD_F64 ? (const void*)g->d_w64[op] : (const void*)g->d_w32[op]))
         return set_error(ctx, RBFFD_ERR_STATE, "weights of operator bit %d not computed", op);
+    std::lock_guard<std::mutex> lk(g->apply_mu);
     // a result written over the field (or part of it): from a copy
     const size_t bytes = (size_t)g->N * ntracers * (dtype == RBFFD_F64 ? 8 : 4);
     void* copy = nullptr;

@@ -119,6 +119,7 @@ struct rbffd_grid {
     int* d_idx_caller = nullptr;
     int wide_applies = 0;
     double* d_field[3] = {nullptr, nullptr, nullptr};
+    std::mutex apply_mu;  // one call at a time uses them
     struct WeightsWork* ww = nullptr;   // the weight solver's device workspace and captured launch (weights.cu)
     size_t bytes = 0;
 };
