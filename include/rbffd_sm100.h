@@ -74,7 +74,8 @@ const char* rbffd_ctx_last_error(const rbffd_ctx* ctx);
 /* Waits for the context's stream.  RBFFD_ERR_TIMEOUT while a PDE of the context
  * holds a state that an advance left when it gave up waiting (rbffd_pde_advance). */
 int rbffd_ctx_synchronize(rbffd_ctx* ctx);
-/* Bytes this context holds on the device, and the device's free/total bytes. */
+/* Bytes this context holds on the device, without the buffers it keeps between
+ * calls (they give way to its other allocations), and the device's free/total bytes. */
 int rbffd_ctx_mem_info(rbffd_ctx* ctx, size_t* held, size_t* free_bytes, size_t* total_bytes);
 /* The context's CUDA stream (cudaStream_t), for callers that order their own work after ours. */
 int rbffd_ctx_stream(rbffd_ctx* ctx, void** stream);

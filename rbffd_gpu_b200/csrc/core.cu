@@ -63,6 +63,10 @@ int dev_alloc(rbffd_ctx* ctx, void** p, size_t bytes)
     *p = nullptr;
     if (bytes == 0) return RBFFD_OK;
     cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx_trim(ctx) > 0) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
     if (e != cudaSuccess) {
         *p = nullptr;
         return cuda_error(ctx, e, "cudaMalloc");
@@ -78,6 +82,69 @@ void dev_free(rbffd_ctx* ctx, void* p, size_t bytes)
     cudaFree(p);
     std::lock_guard<std::mutex> lk(ctx->mu);
     ctx->held -= std::min(ctx->held, bytes);
+}
+
+void* keep_take(rbffd_ctx* ctx, Kept* k, size_t bytes)
+{
+    {
+        std::lock_guard<std::mutex> lk(ctx->kept_mu);
+        if (!k->listed) ctx->kept.push_back(k);
+        k->listed = k->busy = true;
+        if (k->bytes >= bytes) return k->p;
+        dev_free(ctx, k->p, k->bytes);
+        k->p = nullptr;
+        k->bytes = 0;
+    }
+    void* p = nullptr;
+    const int rc = dev_alloc(ctx, &p, bytes);
+    std::lock_guard<std::mutex> lk(ctx->kept_mu);
+    k->p = p;
+    k->bytes = rc == RBFFD_OK ? bytes : 0;
+    return p;
+}
+
+void keep_release(rbffd_ctx* ctx, Kept* k)
+{
+    std::lock_guard<std::mutex> lk(ctx->kept_mu);
+    k->busy = false;
+}
+
+void keep_free(rbffd_ctx* ctx, Kept* k)
+{
+    std::lock_guard<std::mutex> lk(ctx->kept_mu);
+    ctx->kept.erase(std::remove(ctx->kept.begin(), ctx->kept.end(), k), ctx->kept.end());
+    dev_free(ctx, k->p, k->bytes);
+    *k = Kept{};
+}
+
+size_t ctx_kept(rbffd_ctx* ctx)
+{
+    std::lock_guard<std::mutex> lk(ctx->kept_mu);
+    size_t sum = 0;
+    for (const Kept* k : ctx->kept)
+        if (!k->busy) sum += k->bytes;
+    return sum;
+}
+
+size_t ctx_in_use(rbffd_ctx* ctx)
+{
+    const size_t kept = ctx_kept(ctx);
+    std::lock_guard<std::mutex> lk(ctx->mu);
+    return ctx->held - std::min(ctx->held, kept);
+}
+
+size_t ctx_trim(rbffd_ctx* ctx)
+{
+    std::lock_guard<std::mutex> lk(ctx->kept_mu);
+    size_t sum = 0;
+    for (Kept* k : ctx->kept)
+        if (!k->busy && k->p) {
+            sum += k->bytes;
+            dev_free(ctx, k->p, k->bytes);
+            k->p = nullptr;
+            k->bytes = 0;
+        }
+    return sum;
 }
 
 extern "C" const char* rbffd_version(void) { return RBFFD_VERSION_STRING; }
@@ -168,7 +235,7 @@ extern "C" int rbffd_ctx_destroy(rbffd_ctx* ctx)
     cudaStreamDestroy(ctx->stream);
     if (ctx->d_status) cudaFree(ctx->d_status);
     for (int* p : ctx->wait_pages) cudaFreeHost(p);
-    if (ctx->stage) cudaFree(ctx->stage);
+    keep_free(ctx, &ctx->stage);
     delete ctx;
     return RBFFD_OK;
 }
@@ -222,10 +289,7 @@ extern "C" int rbffd_ctx_mem_info(rbffd_ctx* ctx, size_t* held, size_t* free_byt
     cudaSetDevice(ctx->device);
     size_t f = 0, t = 0;
     RBFFD_CUDA_TRY(ctx, cudaMemGetInfo(&f, &t));
-    if (held) {
-        std::lock_guard<std::mutex> lk(ctx->mu);
-        *held = ctx->held;
-    }
+    if (held) *held = ctx_in_use(ctx);
     if (free_bytes) *free_bytes = f;
     if (total_bytes) *total_bytes = t;
     return RBFFD_OK;
@@ -394,8 +458,8 @@ extern "C" int rbffd_grid_destroy(rbffd_grid* g)
     resident_free(g);
     for (auto& kv : g->halos) halo_free(g, kv.second);
     if (g->whole) halo_free(g, g->whole);
-    for (int k = 0; k < 3; k++) dev_free(ctx, g->d_field[k], (k < 2 ? 1 : 2) * (size_t)g->N * sizeof(double));
-    dev_free(ctx, g->d_idx_caller, wsz * sizeof(int));
+    for (Kept& f : g->field) keep_free(ctx, &f);
+    keep_free(ctx, &g->idx_caller);
     delete g;
     return RBFFD_OK;
 }
@@ -1009,7 +1073,9 @@ int grid_permute_preload()
 extern "C" int rbffd_grid_nbytes(const rbffd_grid* g, size_t* bytes)
 {
     if (!g || !bytes) return RBFFD_ERR_INVALID;
-    *bytes = g->bytes;
+    std::lock_guard<std::mutex> lk(g->ctx->kept_mu);
+    *bytes = g->bytes + g->idx_caller.bytes;
+    for (const Kept& f : g->field) *bytes += f.bytes;
     return RBFFD_OK;
 }
 
@@ -1125,26 +1191,10 @@ int grid_alloc_w64(rbffd_grid* g, int op)
 }
 
 // The context's staging buffer for weights on their way in or out, of the size
-// asked for up to STAGE_MAX (larger moves go in parts), kept until the context
-// ends.  The caller holds ctx->stage_mu and has finished its use of the buffer
-// when it lets go.  An allocation per call took longer than the move itself
-// (0.3 ms at 1 MB).
+// asked for up to STAGE_MAX (larger moves go in parts), kept between calls (Kept).
+// The caller holds ctx->stage_mu and has finished its use of the buffer when it
+// lets go.  An allocation per call took longer than the move itself (0.3 ms at 1 MB).
 constexpr size_t STAGE_MAX = (size_t)16 << 20;
-static int ctx_stage(rbffd_ctx* ctx, size_t want, double** buf, size_t* bytes)
-{
-    want = std::min(want, STAGE_MAX);
-    if (ctx->stage_bytes < want) {
-        dev_free(ctx, ctx->stage, ctx->stage_bytes);
-        ctx->stage = nullptr;
-        ctx->stage_bytes = 0;
-        const int rc = dev_alloc(ctx, (void**)&ctx->stage, want);
-        if (rc) return rc;
-        ctx->stage_bytes = want;
-    }
-    *buf = ctx->stage;
-    *bytes = ctx->stage_bytes;
-    return RBFFD_OK;
-}
 
 // Move one operator's weights between the host layout and w64: in parts of whole rows.
 static int weights_move(rbffd_grid* g, double* w64, const double* in, double* out)
@@ -1153,11 +1203,12 @@ static int weights_move(rbffd_grid* g, double* w64, const double* in, double* ou
     cudaStream_t s = ctx->stream;
     std::lock_guard<std::mutex> lk(ctx->stage_mu);
     const size_t row = (size_t)g->n_pad * sizeof(double);
-    double* stage = nullptr;
-    size_t bytes = 0;
-    const int rc = ctx_stage(ctx, (size_t)g->N * row, &stage, &bytes);
-    if (rc) return rc;
-    const int part = (int)std::min<size_t>((size_t)g->N, bytes / row);
+    double* const stage = (double*)keep_take(ctx, &ctx->stage, std::min((size_t)g->N * row, STAGE_MAX));
+    if (!stage) {
+        keep_release(ctx, &ctx->stage);
+        return RBFFD_ERR_OOM;
+    }
+    const int part = (int)std::min<size_t>((size_t)g->N, ctx->stage.bytes / row);
     const unsigned nb = (unsigned)(((size_t)g->N32 * g->nc + 255) / 256);
     cudaError_t e = cudaSuccess;
     for (int c0 = 0; e == cudaSuccess && c0 < g->N; c0 += part) {
@@ -1175,6 +1226,7 @@ static int weights_move(rbffd_grid* g, double* w64, const double* in, double* ou
         }
     }
     const cudaError_t f = cudaStreamSynchronize(s);
+    keep_release(ctx, &ctx->stage);
     if (e == cudaSuccess) e = f;
     return e == cudaSuccess ? RBFFD_OK : cuda_error(ctx, e, in ? "rbffd_weights_set" : "rbffd_weights_get");
 }
@@ -1355,16 +1407,22 @@ __global__ void k_caller_index(const int4* __restrict__ idx, const int* __restri
 // nullptr before that, and if there is no memory for them.
 static const int* grid_caller_index(rbffd_grid* g)
 {
-    if (g->d_idx_caller || ++g->wide_applies < 16) return g->d_idx_caller;
     const size_t n = (size_t)g->N32 * g->n4;
-    if (dev_alloc(g->ctx, (void**)&g->d_idx_caller, n * sizeof(int)) != RBFFD_OK) {
-        g->wide_applies = 0;  // asked for again later
-        return nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g->ctx->kept_mu);
+        if (g->idx_caller.p) {
+            g->idx_caller.busy = true;
+            return (const int*)g->idx_caller.p;
+        }
     }
-    g->bytes += n * sizeof(int);
-    k_caller_index<<<(unsigned)((n / 4 + 255) / 256), 256, 0, g->ctx->stream>>>((const int4*)g->d_idx, g->d_perm, n / 4,
-                                                                               (int4*)g->d_idx_caller);
-    return g->d_idx_caller;
+    if (g->wide_applies == 16) g->wide_applies = 0;  // not had, or given back: asked for again later
+    if (++g->wide_applies < 16) return nullptr;
+    KeepError keep(g->ctx);
+    int* const p = (int*)keep_take(g->ctx, &g->idx_caller, n * sizeof(int));
+    if (p)
+        k_caller_index<<<(unsigned)((n / 4 + 255) / 256), 256, 0, g->ctx->stream>>>((const int4*)g->d_idx, g->d_perm,
+                                                                                   n / 4, (int4*)p);
+    return p;
 }
 
 template <typename T, typename U, bool PLAIN, bool THROUGH>
@@ -1386,10 +1444,21 @@ static void launch_apply_caller_t(rbffd_grid* g, const int* idx, const T* w, con
 // grids up to 65536 nodes stay with small allocations); nullptr without memory.
 static double* grid_field(rbffd_grid* g, int k)
 {
-    const size_t bytes = (k < 2 ? 1 : 2) * (size_t)g->N * sizeof(double);
-    if (!g->d_field[k] && dev_alloc(g->ctx, (void**)&g->d_field[k], bytes) == RBFFD_OK) g->bytes += bytes;
-    return g->d_field[k];
+    return (double*)keep_take(g->ctx, &g->field[k], (k < 2 ? 1 : 2) * (size_t)g->N * sizeof(double));
 }
+
+// A call's use of the grid's kept buffers, one call at a time; it ends with the call's work done.
+struct ApplyUse {
+    rbffd_grid* g;
+    std::lock_guard<std::mutex> lk;
+    explicit ApplyUse(rbffd_grid* q) : g(q), lk(q->apply_mu) {}
+    ~ApplyUse()
+    {
+        std::lock_guard<std::mutex> l2(g->ctx->kept_mu);
+        for (Kept& f : g->field) f.busy = false;
+        g->idx_caller.busy = false;
+    }
+};
 
 // Node records of at most half a 32-byte sector: on grids past 65536 nodes the
 // field is reordered first, since the caller's order spreads a row's neighbours
@@ -1404,6 +1473,7 @@ static void launch_apply_caller(rbffd_grid* g, const T* w, const U* u, U* out, i
     if (T_tr * sizeof(U) > 16) {
         idx = grid_caller_index(g);
     } else if (g->N > 65536) {
+        KeepError keep(g->ctx);
         U* const ui = (U*)grid_field(g, 2);
         if (ui && grid_to_internal(g, u, ui, T_tr, sizeof(U), s) == RBFFD_OK) {
             idx = g->d_idx;
@@ -1457,7 +1527,7 @@ extern "C" int rbffd_apply(rbffd_grid* g, unsigned der_type, int dtype, unsigned
     rbffd_ctx* ctx = g->ctx;
     cudaSetDevice(ctx->device);
     int N = g->N;
-    std::lock_guard<std::mutex> lk(g->apply_mu);
+    ApplyUse use(g);
     // the field and its derivative on the device, in the caller's order; kept with the grid
     const size_t b64 = (size_t)N * sizeof(double);
     double *const du = grid_field(g, 0), *const dd = grid_field(g, 1);
@@ -1489,7 +1559,7 @@ extern "C" int rbffd_apply_dev(rbffd_grid* g, unsigned der_type, int dtype, int 
     cudaStream_t s = ctx->stream;
     if (!(dtype == RBFFD_F64 ? (const void*)g->d_w64[op] : (const void*)g->d_w32[op]))
         return set_error(ctx, RBFFD_ERR_STATE, "weights of operator bit %d not computed", op);
-    std::lock_guard<std::mutex> lk(g->apply_mu);
+    ApplyUse use(g);
     // a result written over the field (or part of it): from a copy
     const size_t bytes = (size_t)g->N * ntracers * (dtype == RBFFD_F64 ? 8 : 4);
     void* copy = nullptr;

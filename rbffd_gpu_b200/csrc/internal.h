@@ -48,6 +48,15 @@ struct Shape {
 // nonzero code here instead of hanging or trapping; the host reads and clears it.
 enum { DEV_STATUS_OK = 0, DEV_STATUS_WAIT_TIMEOUT = 1 };
 
+// A device buffer kept between calls.  One that no call is using is given back
+// when another allocation of the context fails or its server's budget is short
+// (ctx_trim), and made again when it is next used.
+struct Kept {
+    void* p = nullptr;
+    size_t bytes = 0;
+    bool busy = false, listed = false;
+};
+
 struct rbffd_ctx {
     int device = 0;
     int sm_count = 0;
@@ -60,9 +69,10 @@ struct rbffd_ctx {
     int* d_status = nullptr;         // DEV_STATUS_* written by kernels with bounded waits
     int arith = 0;                   // RBFFD_ARITH_*: FP64 arithmetic of rbffd_apply* and of new FP64 PDEs
     int weights_elim = 0;            // RBFFD_ELIM_*: elimination of the weight solves (0: the default)
-    double* stage = nullptr;         // weights on their way in or out (core.cu), under stage_mu
-    size_t stage_bytes = 0;
+    Kept stage;                      // weights on their way in or out (core.cu), under stage_mu
     std::mutex stage_mu;
+    std::vector<Kept*> kept;         // the context's and its grids' kept buffers; they too are under kept_mu
+    std::mutex kept_mu;
     // Host-mapped DEV_STATUS_* words of the device-resident RK4, one per PDE
     // (ctx_wait_slot), in pages of WAIT_PAGE; under mu
     std::vector<int*> wait_pages, wait_free;
@@ -116,9 +126,8 @@ struct rbffd_grid {
     unsigned short* d_res_lidx = nullptr;   // [res_C][n4][res_R]
     // rbffd_apply*: d_idx in the caller's node numbers (made at the 16th application
     // to wide records), and fields kept between calls (grid_field, core.cu)
-    int* d_idx_caller = nullptr;
+    Kept idx_caller, field[3];
     int wide_applies = 0;
-    double* d_field[3] = {nullptr, nullptr, nullptr};
     std::mutex apply_mu;  // one call at a time uses them
     struct WeightsWork* ww = nullptr;   // the weight solver's device workspace and captured launch (weights.cu)
     size_t bytes = 0;
@@ -257,6 +266,17 @@ size_t pde_bytes(const rbffd_grid* g, const rbffd_pde_params* prm);
 // Advection coefficients of an advection right-hand side, internal node order,
 // in prm->dtype, into device arrays of N values (rk4.cu).
 int advect_coefficients(rbffd_grid* g, const rbffd_pde_params* prm, void* cu_dev, void* cv_dev, cudaStream_t s);
+
+// k's buffer of at least `bytes`, kept or new, in use until keep_release; nullptr
+// without memory.  keep_free: the buffer and its place in the context's list go.
+void* keep_take(rbffd_ctx* ctx, Kept* k, size_t bytes);
+void keep_release(rbffd_ctx* ctx, Kept* k);
+void keep_free(rbffd_ctx* ctx, Kept* k);
+// Frees the kept buffers that are not in use, and returns / returns only their bytes.
+size_t ctx_trim(rbffd_ctx* ctx);
+size_t ctx_kept(rbffd_ctx* ctx);
+// Bytes held without those.
+size_t ctx_in_use(rbffd_ctx* ctx);
 
 // ---- error helpers --------------------------------------------------------
 int set_error(rbffd_ctx* ctx, int status, const char* fmt, ...);

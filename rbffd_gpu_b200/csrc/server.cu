@@ -691,6 +691,12 @@ void admission_loop(rbffd_server* S)
             }
         const size_t need = io_bytes + (bank ? 0 : bank_bytes(g, r->p.pde));
         if (ctx_held(S->ctx) + need > S->budget) {
+            if (ctx_kept(S->ctx) > 0) {  // buffers kept between calls go first
+                lk.unlock();
+                ctx_trim(S->ctx);
+                lk.lock();
+                if (ctx_kept(S->ctx) == 0) continue;
+            }
             size_t k = S->banks.size();  // the idle bank that has been idle longest
             for (size_t q = 0; q < S->banks.size(); q++)
                 if (S->banks[q].get() != bank && S->banks[q]->members == 0 && !S->banks[q]->in_plan &&
@@ -729,6 +735,10 @@ void admission_loop(rbffd_server* S)
         double* io = nullptr;
         if (rc == RBFFD_OK) {
             cudaError_t e = cudaMallocAsync((void**)&io, io_bytes, S->astream);
+            if (e == cudaErrorMemoryAllocation && ctx_trim(S->ctx) > 0) {
+                cudaGetLastError();
+                e = cudaMallocAsync((void**)&io, io_bytes, S->astream);
+            }
             if (e == cudaSuccess) e = cudaMemcpyAsync(io, r->u0.data(), io_bytes, cudaMemcpyHostToDevice, S->astream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(S->astream);
             if (e != cudaSuccess) {
@@ -1326,7 +1336,7 @@ extern "C" int rbffd_server_submit(rbffd_server* S, const rbffd_request* req, ui
     std::lock_guard<std::mutex> lk(S->mu);
     if (S->stop) return set_error(ctx, RBFFD_ERR_STATE, "server is stopping");
     // memory the server cannot free (grids, the caller's own PDEs) plus this request
-    const size_t held = ctx_held(ctx);
+    const size_t held = ctx_in_use(ctx);
     if (held - std::min(held, S->owned) + need > S->budget)
         return set_error(ctx, RBFFD_ERR_BUDGET, "request needing %zu bytes can never fit the budget of %zu bytes", need,
                          S->budget);
@@ -1410,7 +1420,7 @@ extern "C" int rbffd_server_get_stats(rbffd_server* S, rbffd_server_stats* out)
     *out = S->st;
     out->pending = (long long)S->pending.size();
     out->active = (long long)(S->active.size() + S->ready.size()) + S->finishing;
-    out->held_bytes = (double)ctx_held(S->ctx);
+    out->held_bytes = (double)ctx_in_use(S->ctx);
     return RBFFD_OK;
 }
 
