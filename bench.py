@@ -315,13 +315,13 @@ def e2e_heat(R, ctx, pde, u0, nsteps, ws):
     return replicas_max(time.perf_counter() - t, ws), oh.copy()
 
 
-def device_resident(shape):
-    """The shape an advance reports when its steps ran device-resident (rbffd_pde_advance)."""
-    return tuple(shape) == (1, 256, 0)
+def device_resident(pde):
+    """Whether the last advance ran device-resident (rbffd_pde_get_path)."""
+    return pde.getPath()[0] == pde.PATH_RESIDENT
 
 
-def stage_kernel_name(shape, tname):
-    if device_resident(shape):
+def stage_kernel_name(shape, tname, resident):
+    if resident:
         return "k_rk4_grid<%s,HEAT> (every step of an advance in one cooperative launch, 16-bit local indices)" % tname
     if shape[2] > 0:
         return "k_stage_tile<%s,HEAT> (halo tile of %d rows, 16-bit local indices)" % (tname, shape[2])
@@ -386,10 +386,9 @@ def run_ours(args):
         tot_ms, step_ms = timed_heat_steps(torch, ctx, pde, args.steps, flush, ws, clocks)
         clk = clocks.stop()
         shape = pde.getShape()  # (lanes per row, threads per block, rows per halo tile or 0): the path's or the tuner's pick
-        resident = device_resident(shape)
+        resident = device_resident(pde)
         stages = 4 * steps * args.steps
-        # device-resident: one launch per 2000 steps of an advance; else one fused stage kernel per RK4 stage
-        launches = args.steps * -(-steps // 2000) if resident else stages
+        launches = args.steps * pde.getPath()[1]
         per_stage_s = tot_ms * 1e-3 / stages
         tiled = resident or shape[2] > 0
         bytes_launch = N * stage_bytes(n, wb, wb, 2 if tiled else 4)
@@ -399,10 +398,11 @@ def run_ours(args):
         res[tag] = {
             "value": replicas_rate(float(N) * steps * args.steps, ws, tot_ms * 1e-3), "ms_per_step": tot_ms / args.steps,
             "launches": launches, "clocks": clk, "shape": shape, "u_final": pde.getLocalSolution(),
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+            "roofline": {"bound": "on-chip (shared memory and L2)" if resident else "hbm", "achieved": achieved,
+                         "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": None if resident else stage_traffic(tag[:4].replace("fp", "f"), tiled),
                          "peak_kind": peak_kind,
-                         "kernel": stage_kernel_name(shape, "double" if wb == 8 else "float") +
+                         "kernel": stage_kernel_name(shape, "double" if wb == 8 else "float", resident) +
                          ", fused SpMV + RHS + RK4 stage", "shape": shape, "algorithmic_bytes_per_stage": bytes_launch,
                          "l2_resident": True,
                          "note": "per-stage time = timed region / stages. The %s weights and indices (%.1f MB) stay on "

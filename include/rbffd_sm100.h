@@ -422,6 +422,15 @@ enum rbffd_advance_flags {
  * graph, RBFFD_ADVANCE_ASYNC calls record their stage launches, without a shape
  * set or tuned before with one lane per row. */
 int rbffd_pde_advance(rbffd_pde* pde, int scheme, double dt, int nsteps, int flags);
+/* How the PDE's last advance ran, and (launches, may be NULL) in how many kernel launches. */
+enum rbffd_advance_path {
+    RBFFD_PATH_NONE = 0,     /* none yet */
+    RBFFD_PATH_STAGES = 1,   /* one launch per stage */
+    RBFFD_PATH_RESIDENT = 2, /* device-resident: cooperative launches of many steps */
+    RBFFD_PATH_CLUSTER = 3,  /* RBFFD_ADVANCE_RESIDENT: one launch of a thread-block cluster */
+    RBFFD_PATH_UNFUSED = 4   /* RBFFD_ADVANCE_UNFUSED */
+};
+int rbffd_pde_get_path(rbffd_pde* pde, int* path, int* launches);
 /* Polls a block of the device-resident RK4 makes for a neighbour's value before
  * it gives up (default 2^21, about a second); 0: gives up on any wait. */
 int rbffd_pde_set_poll_limit(rbffd_pde* pde, int polls);

@@ -637,6 +637,14 @@ class TimeDependentPDE:
         self.ctx.check(self.ctx.L.rbffd_pde_get_time(self.h, ctypes.byref(t)))
         return t.value
 
+    PATH_NONE, PATH_STAGES, PATH_RESIDENT, PATH_CLUSTER, PATH_UNFUSED = 0, 1, 2, 3, 4
+
+    def getPath(self):
+        """How the last advance ran (PATH_*) and in how many kernel launches (rbffd_pde_get_path)."""
+        p, n = ctypes.c_int(), ctypes.c_int()
+        self.ctx.check(self.ctx.L.rbffd_pde_get_path(self.h, ctypes.byref(p), ctypes.byref(n)))
+        return p.value, n.value
+
     def setPollLimit(self, polls):
         """Polls a block of the device-resident RK4 makes for a neighbour's value
         before it gives up (rbffd_pde_set_poll_limit)."""

@@ -492,6 +492,13 @@ public:
         return u;
     }
     void setTime(double t) { check(ctx(), rbffd_pde_set_time(h_, t), "setTime"); }
+    // how the last advance ran (rbffd_advance_path)
+    int getPath()
+    {
+        int p = 0;
+        check(ctx(), rbffd_pde_get_path(h_, &p, nullptr), "getPath");
+        return p;
+    }
     // polls of the device-resident RK4 before a wait gives up (rbffd_pde_set_poll_limit)
     void setPollLimit(int polls) { check(ctx(), rbffd_pde_set_poll_limit(h_, polls), "setPollLimit"); }
     // FP32 PDEs: carry each step's rounding of u + increment into the next (rbffd_pde_set_compensated_state)

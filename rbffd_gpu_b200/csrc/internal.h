@@ -243,10 +243,11 @@ struct rbffd_pde {
     Shape shape;
     bool forced = false;
     // Device-resident RK4 (rk4_grid.cuh): stage inputs with their stage numbers (two
-    // buffers, by parity), the next stage number, and whether the last advance ran there
+    // buffers, by parity), the next stage number
     void* word = nullptr;
     unsigned word_tag = 1;
-    bool on_grid = false, one_lane = false;  // one_lane: or per stage with its bits
+    bool one_lane = false;  // the last advance ran there, at least in part, or per stage with its bits
+    int path = 0, launches = 0;  // of the last advance: RBFFD_PATH_*, and its kernel launches
     // Its bounded waits: the status word (host-mapped) a launch that gave up leaves
     // DEV_STATUS_WAIT_TIMEOUT in until the state is set again, the polls a wait
     // makes, and the time up to which the steps are known to be complete

@@ -1972,16 +1972,28 @@ extern "C" int rbffd_pde_set_tiled_shape(rbffd_pde* P, int rows_per_block, int l
 extern "C" int rbffd_pde_get_tiling(rbffd_pde* P, int* rows_per_block)
 {
     if (!P || !rows_per_block) return RBFFD_ERR_INVALID;
-    *rows_per_block = P->shape.tile;
+    *rows_per_block = !P->forced && P->one_lane ? 0 : P->shape.tile;
     return RBFFD_OK;
 }
 
 extern "C" int rbffd_pde_get_tile_flags(rbffd_pde* P, int* flags)
 {
     if (!P || !flags) return RBFFD_ERR_INVALID;
+    if (!P->forced && P->one_lane) {
+        *flags = 0;
+        return RBFFD_OK;
+    }
     *flags = (P->shape.tma ? RBFFD_TILE_STREAM_WEIGHTS : 0) | (P->shape.sched ? RBFFD_TILE_SLOT_SCHEDULE : 0) |
              (P->shape.pf ? RBFFD_TILE_PREFETCH : 0) | (P->shape.pipe ? RBFFD_TILE_PIPELINE : 0) |
              (P->shape.db ? RBFFD_TILE_DOUBLE_BUFFER : 0);
+    return RBFFD_OK;
+}
+
+extern "C" int rbffd_pde_get_path(rbffd_pde* P, int* path, int* launches)
+{
+    if (!P || !path) return RBFFD_ERR_INVALID;
+    *path = P->path;
+    if (launches) *launches = P->launches;
     return RBFFD_OK;
 }
 
@@ -2148,6 +2160,8 @@ static int advance_resident(rbffd_pde* P, double dt, int nsteps, int flags)
     const int rc = P->dtype == RBFFD_F64 ? advance_resident_t<double>(P, dt, nsteps, s, false)
                                          : advance_resident_t<float>(P, dt, nsteps, s, false);
     if (rc) return rc;
+    P->path = RBFFD_PATH_CLUSTER;
+    P->launches = 1;
     P->t += dt * nsteps;
     if (!(flags & RBFFD_ADVANCE_ASYNC)) return pde_synchronize(P);
     return RBFFD_OK;
@@ -2363,6 +2377,7 @@ static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const Gri
         });
         if (e != cudaSuccess) return e;
         P->word_tag += 4u * (unsigned)gp.nsteps;
+        P->launches++;
         *done += gp.nsteps;
     }
     return cudaSuccess;
@@ -2415,6 +2430,8 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
     cudaStream_t s = ctx->stream;
     if (flags & RBFFD_ADVANCE_UNFUSED) {
         // plain path: per-operator SpMV launches, separate RHS/axpy, host sync per step
+        P->path = RBFFD_PATH_UNFUSED;
+        P->launches = 0;
         size_t n = (size_t)P->g->N * P->T * (P->dtype == RBFFD_F64 ? 8 : 4);
         int nops = P->kind == KIND_HEAT ? 1 : (P->use_hv ? 3 : 2);
         for (int k = 0; k < nops; k++)
@@ -2426,6 +2443,7 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
         for (int k = 0; k < nsteps; k++) {
             for (int st = 0; st < 4; st++) {
                 int rc = P->dtype == RBFFD_F64 ? unfused_stage<double>(P, st, dt, s) : unfused_stage<float>(P, st, dt, s);
+                P->launches += nops + 1;
                 if (rc) return rc;
             }
             P->t += dt;
@@ -2439,14 +2457,16 @@ extern "C" int rbffd_pde_advance(rbffd_pde* P, int scheme, double dt, int nsteps
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     RBFFD_CUDA_TRY(ctx, cudaStreamIsCapturing(s, &cap));
     const bool capturing = cap != cudaStreamCaptureStatusNone;
+    P->launches = 0;
     const int done = P->forced || capturing ? 0 : advance_grid(P, dt, nsteps);
-    P->on_grid = done == nsteps;
+    P->path = done == nsteps ? RBFFD_PATH_RESIDENT : RBFFD_PATH_STAGES;
     P->one_lane = done > 0 || (capturing && !P->forced && P->shape.block == 0 && P->shape.tile == 0);
-    if (P->on_grid) {
+    if (done == nsteps) {
         P->t += dt * nsteps;
         return flags & RBFFD_ADVANCE_ASYNC ? RBFFD_OK : pde_synchronize(P);
     }
     const int left = nsteps - done;
+    P->launches += 4 * left;
     if (!P->forced && !P->one_lane && P->shape.block == 0 && P->shape.tile == 0) P->shape = autotune(P);
     Shape sh = P->one_lane ? Shape{1, 256} : P->shape;  // the rest of a call with the same bits
     if (sh.tile > 0) {  // the halo must exist before any capture (building it copies to the device)

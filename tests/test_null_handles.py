@@ -4,3 +4,7 @@ from rbffd_gpu_b200 import _lib
 
 def test_poll_limit():
     assert _lib.load().rbffd_pde_set_poll_limit(None, 1) == -1
+
+
+def test_path():
+    assert _lib.load().rbffd_pde_get_path(None, None, None) == -1
