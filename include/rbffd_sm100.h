@@ -415,7 +415,7 @@ enum rbffd_advance_flags {
  * is lost: the call returns RBFFD_ERR_TIMEOUT, or with RBFFD_ADVANCE_ASYNC the
  * next rbffd_ctx_synchronize, rbffd_pde_get_state or rbffd_pde_advance that finds
  * it ended does, and these calls on the PDE go on to until rbffd_pde_set_state
- * gives it a new state.  Steps issued meanwhile do not run, and the PDE's time
+ * gives it a new state.  Steps issued meanwhile are lost too, and the PDE's time
  * returns to that of the last steps known to be complete.  Other PDEs are not
  * affected.
  * While the caller captures the context's stream (rbffd_ctx_stream) in a CUDA
@@ -431,9 +431,9 @@ enum rbffd_advance_path {
     RBFFD_PATH_UNFUSED = 4   /* RBFFD_ADVANCE_UNFUSED */
 };
 int rbffd_pde_get_path(rbffd_pde* pde, int* path, int* launches);
-/* Polls a block of the device-resident RK4 makes for a neighbour's value before
- * it gives up (default 2^21, about a second); 0: gives up on any wait. */
-int rbffd_pde_set_poll_limit(rbffd_pde* pde, int polls);
+/* Fault injection: while on, a block of the device-resident RK4 gives up at its
+ * first wait as if it had run out (about a second). */
+int rbffd_pde_inject_wait_failure(rbffd_pde* pde, int on);
 /* Heat-equation RK4 that allocates no device memory.  No counterpart in the
  * reference: it exists for callers that cannot let a library allocate on the
  * GPU -- applications that reserve the device's memory for their own pool, or

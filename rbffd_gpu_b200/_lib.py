@@ -98,7 +98,7 @@ PROTOTYPES = {
     "rbffd_pde_get_time": (c_int, [c_void_p, dp]),
     "rbffd_pde_advance": (c_int, [c_void_p, c_int, c_double, c_int, c_int]),
     "rbffd_pde_get_path": (c_int, [c_void_p, ip, ip]),
-    "rbffd_pde_set_poll_limit": (c_int, [c_void_p, c_int]),
+    "rbffd_pde_inject_wait_failure": (c_int, [c_void_p, c_int]),
     "rbffd_pde_set_shape": (c_int, [c_void_p, c_int, c_int]),
     "rbffd_pde_set_arithmetic": (c_int, [c_void_p, c_int]),
     "rbffd_pde_get_arithmetic": (c_int, [c_void_p, ip]),

@@ -645,10 +645,10 @@ class TimeDependentPDE:
         self.ctx.check(self.ctx.L.rbffd_pde_get_path(self.h, ctypes.byref(p), ctypes.byref(n)))
         return p.value, n.value
 
-    def setPollLimit(self, polls):
-        """Polls a block of the device-resident RK4 makes for a neighbour's value
-        before it gives up (rbffd_pde_set_poll_limit)."""
-        self.ctx.check(self.ctx.L.rbffd_pde_set_poll_limit(self.h, int(polls)), "set_poll_limit")
+    def injectWaitFailure(self, on=True):
+        """While on, a block of the device-resident RK4 gives up at its first wait
+        (rbffd_pde_inject_wait_failure)."""
+        self.ctx.check(self.ctx.L.rbffd_pde_inject_wait_failure(self.h, int(bool(on))), "inject_wait_failure")
 
     def setShape(self, lanes_per_row=0, block_threads=0):
         self.ctx.check(self.ctx.L.rbffd_pde_set_shape(self.h, lanes_per_row, block_threads), "set_shape")

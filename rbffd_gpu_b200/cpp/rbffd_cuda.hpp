@@ -499,8 +499,8 @@ public:
         check(ctx(), rbffd_pde_get_path(h_, &p, nullptr), "getPath");
         return p;
     }
-    // polls of the device-resident RK4 before a wait gives up (rbffd_pde_set_poll_limit)
-    void setPollLimit(int polls) { check(ctx(), rbffd_pde_set_poll_limit(h_, polls), "setPollLimit"); }
+    // while on, a device-resident advance gives up at its first wait (rbffd_pde_inject_wait_failure)
+    void injectWaitFailure(bool on) { check(ctx(), rbffd_pde_inject_wait_failure(h_, on ? 1 : 0), "injectWaitFailure"); }
     // FP32 PDEs: carry each step's rounding of u + increment into the next (rbffd_pde_set_compensated_state)
     void setCompensatedState(bool on) { check(ctx(), rbffd_pde_set_compensated_state(h_, on ? 1 : 0), "setCompensatedState"); }
     // PDE::checkLocalError (pde.h:120-127): the solution's error norms against

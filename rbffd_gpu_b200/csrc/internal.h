@@ -249,10 +249,10 @@ struct rbffd_pde {
     bool one_lane = false;  // the last advance ran there, at least in part, or per stage with its bits
     int path = 0, launches = 0;  // of the last advance: RBFFD_PATH_*, and its kernel launches
     // Its bounded waits: the status word (host-mapped) a launch that gave up leaves
-    // DEV_STATUS_WAIT_TIMEOUT in until the state is set again, the polls a wait
-    // makes, and the time up to which the steps are known to be complete
+    // DEV_STATUS_WAIT_TIMEOUT in until the state is set again, whether the next
+    // launches give up, and the time up to which the steps are known to be complete
     int* wait = nullptr;
-    int poll_limit = 1 << 21;
+    int inject_wait = 0;
     double t_sure = 0.0;
     int grid_skip = 0;  // advances left before memory it did not get is asked for again
     int arith = 0;  // RBFFD_ARITH_*

@@ -1863,10 +1863,10 @@ extern "C" int rbffd_pde_get_time(rbffd_pde* P, double* t)
     return RBFFD_OK;
 }
 
-extern "C" int rbffd_pde_set_poll_limit(rbffd_pde* P, int polls)
+extern "C" int rbffd_pde_inject_wait_failure(rbffd_pde* P, int on)
 {
-    if (!P || polls < 0) return RBFFD_ERR_INVALID;
-    P->poll_limit = polls;
+    if (!P) return RBFFD_ERR_INVALID;
+    P->inject_wait = on != 0;
     return RBFFD_OK;
 }
 
@@ -2352,7 +2352,7 @@ static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const Gri
     gp.word[1] = (char*)P->word + 2 * (size_t)g->N * P->T * sizeof(T);
     gp.status = P->wait;  // one address on host and device (unified addressing)
     gp.gave_up = word_gave_up(P);
-    gp.polls = P->poll_limit;
+    gp.fail = P->inject_wait;
     gp.c[0] = gp.c[1] = s0.c;
     gp.c[2] = make_params<T>(P, 2, dt).c;
     gp.c[3] = s3.c;

@@ -18,9 +18,10 @@
 // writes stage s + 2 over stage s only after it has the values of stage s + 1
 // from every CTA that reads it, which those wrote after reading stage s (the
 // host adds a word to the reader's list where only one of two CTAs reads the
-// other).  Waits are bounded (polls); a CTA whose wait runs out marks the launch
-// as given up, on the device and for the host, and ends, as do the others when
-// theirs run out, and every later launch on that state at its start.
+// other).  Waits are bounded (GRID_POLL_LIMIT, a constant: as a parameter it cost
+// stages 3 to 14%); a CTA whose wait runs out marks the launch as given up, on
+// the device and for the host, and ends, as do the others when theirs run out,
+// and every later launch on that state after its first stage.
 //
 // One lane per (row, tracer), slots in stencil order: the arithmetic of
 // k_stage_scalar and k_stage_vec with one lane per row, bit for bit.
@@ -30,6 +31,8 @@
 // ones the shared-memory gathers, and the L2 reads of what does not fit.  The
 // times at which the per-stage kernels lose to it are at grid_geom (rk4.cu).
 #pragma once
+
+constexpr int GRID_POLL_LIMIT = 1 << 21;  // polls of one word (about a second)
 
 template <typename T>
 struct GridParams {
@@ -48,7 +51,7 @@ struct GridParams {
     void* word[2];                 // stage inputs with their stage numbers, by parity
     int* status;                   // host-mapped; DEV_STATUS_WAIT_TIMEOUT on a wait that ran out
     int* gave_up;                  // the same for launches that follow, in device memory
-    int polls;                     // polls of a word before its wait runs out
+    int fail;                      // nonzero: the first wait counts as run out (injected)
     T c[4];                        // dt/2, dt/2, dt, dt/6
     T kappa;
     int nc, T_tr, R, cs, H, nr, nsteps;  // cs: chunks in shared memory; H: halo positions; nr: most words read
@@ -230,7 +233,6 @@ __global__ void __launch_bounds__(MAXT, 1) k_rk4_grid(GridParams<T> gp)
         if (AHEAD && ns > 0) load(rr[q], 0, ahead[q]);
     }
     __syncthreads();
-    if (s_fail) return;  // an earlier launch gave up: its state is not one of a step's
     bool live = false;  // warps without items only take neighbours' values
 #pragma unroll
     for (int q = 0; q < IPT; q++) live |= own[q] >= 0;
@@ -322,20 +324,19 @@ __global__ void __launch_bounds__(MAXT, 1) k_rk4_grid(GridParams<T> gp)
                 }
         if (!publish) break;
         // the neighbours' values of this stage: one word per thread, or four in flight
-        bool late = false;
         const int words = nread * TT;
+        bool late = false;
         if (words <= TH) {
             if (tid < words) {
                 const int k = tid / TT, t = tid - k * TT;
                 const size_t i = (size_t)rn[k] * TT + t;
-                T v = T(0);
-                for (int tries = 0;; tries++) {
-                    if (tries >= gp.polls) {
+                T v;
+                int tries = 0;
+                while (!word_load(word, i, tag, v))
+                    if (++tries > GRID_POLL_LIMIT) {
                         late = true;
                         break;
                     }
-                    if (word_load(word, i, tag, v)) break;
-                }
                 hout[rp[k] * TT + t] = v;
             }
         } else for (int e0 = tid; e0 < words && !late; e0 += 4 * TH) {
@@ -356,7 +357,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_rk4_grid(GridParams<T> gp)
                 }
             }
             for (int tries = 0; wait; tries++) {
-                if (tries >= gp.polls) {
+                if (tries > GRID_POLL_LIMIT) {
                     late = true;
                     break;
                 }
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_rk4_grid(GridParams<T> gp)
                     }
             }
         }
-        if (late) s_fail = 1;
+        if (late || (gp.fail && words > 0)) s_fail = 1;
         __syncthreads();
         if (s_fail) {
             if (tid == 0) {

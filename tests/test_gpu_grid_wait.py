@@ -1,4 +1,4 @@
-"""A device-resident advance whose waits run out (a poll limit of 0): the error
+"""A device-resident advance whose waits run out (injected): the error
 is the advancing PDE's own, reported also after an asynchronous advance, kept
 until the state is set again, and nothing else of the context is affected."""
 import numpy as np
@@ -40,7 +40,7 @@ def test_wait_runs_out(ctx, T, asynchronous):
         p.fillInitialConditions(u0)
         p.advance(R.RK4, DT, 4)
     t = pde.getTime()
-    pde.setPollLimit(0)
+    pde.injectWaitFailure()
     if asynchronous:
         pde.advance(R.RK4, DT, 6, asynchronous=True)
         try:
@@ -61,14 +61,14 @@ def test_wait_runs_out(ctx, T, asynchronous):
     ref.advance(R.RK4, DT, 6)
     assert np.array_equal(other.getLocalSolution(), ref.getLocalSolution())
     assert other.getTime() == ref.getTime()
-    # a new state, the limit back
-    pde.setPollLimit(1 << 21)
+    # a new state, no more failures
+    pde.injectWaitFailure(False)
     pde.fillInitialConditions(u0)
     ctx.synchronize()
     pde.advance(R.RK4, DT, 10)
     assert np.array_equal(pde.getLocalSolution(), ref.getLocalSolution())
     # destroyed while failed: the context is clean again
-    pde.setPollLimit(0)
+    pde.injectWaitFailure()
     expect_timeout(lambda: pde.advance(R.RK4, DT, 1))
     pde.close()
     ctx.synchronize()

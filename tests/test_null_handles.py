@@ -2,8 +2,8 @@
 from rbffd_gpu_b200 import _lib
 
 
-def test_poll_limit():
-    assert _lib.load().rbffd_pde_set_poll_limit(None, 1) == -1
+def test_wait_failure():
+    assert _lib.load().rbffd_pde_inject_wait_failure(None, 1) == -1
 
 
 def test_path():
