@@ -431,8 +431,8 @@ enum rbffd_advance_path {
     RBFFD_PATH_UNFUSED = 4   /* RBFFD_ADVANCE_UNFUSED */
 };
 int rbffd_pde_get_path(rbffd_pde* pde, int* path, int* launches);
-/* Fault injection: while on, a block of the device-resident RK4 gives up at its
- * first wait as if it had run out (about a second). */
+/* Fault injection: while on, the blocks of a device-resident advance wait for
+ * values that nobody publishes, until their waits run out (about a second). */
 int rbffd_pde_inject_wait_failure(rbffd_pde* pde, int on);
 /* Heat-equation RK4 that allocates no device memory.  No counterpart in the
  * reference: it exists for callers that cannot let a library allocate on the

@@ -646,8 +646,8 @@ class TimeDependentPDE:
         return p.value, n.value
 
     def injectWaitFailure(self, on=True):
-        """While on, a block of the device-resident RK4 gives up at its first wait
-        (rbffd_pde_inject_wait_failure)."""
+        """While on, a device-resident advance waits for values that nobody publishes
+        until its waits run out (rbffd_pde_inject_wait_failure)."""
         self.ctx.check(self.ctx.L.rbffd_pde_inject_wait_failure(self.h, int(bool(on))), "inject_wait_failure")
 
     def setShape(self, lanes_per_row=0, block_threads=0):

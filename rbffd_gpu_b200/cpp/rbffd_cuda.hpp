@@ -499,7 +499,7 @@ public:
         check(ctx(), rbffd_pde_get_path(h_, &p, nullptr), "getPath");
         return p;
     }
-    // while on, a device-resident advance gives up at its first wait (rbffd_pde_inject_wait_failure)
+    // while on, a device-resident advance's waits run out (rbffd_pde_inject_wait_failure)
     void injectWaitFailure(bool on) { check(ctx(), rbffd_pde_inject_wait_failure(h_, on ? 1 : 0), "injectWaitFailure"); }
     // FP32 PDEs: carry each step's rounding of u + increment into the next (rbffd_pde_set_compensated_state)
     void setCompensatedState(bool on) { check(ctx(), rbffd_pde_set_compensated_state(h_, on ? 1 : 0), "setCompensatedState"); }

@@ -981,6 +981,7 @@ int grid_halo_whole(rbffd_grid* g, int R, const Halo** out)
     h->nblocks = nblocks;
     h->max_halo = max_halo;
     h->max_read = max_read;
+    h->nread = g->whole_meta[2 * nb1 + nblocks];
     const std::vector<int>& meta = g->whole_meta;
     const size_t nlidx = (size_t)g->N32 * g->n4, nhalo = (size_t)meta[nb1 + nblocks], nread = (size_t)meta[2 * nb1 + nblocks];
     // one allocation: lidx | rpos | rnode | nodes | meta (16-bit arrays of even length first)

@@ -179,7 +179,7 @@ struct Halo {
     int* d_rptr = nullptr;             // [nblocks + 1]
     int* d_rnode = nullptr;
     unsigned short* d_rpos = nullptr;
-    int max_read = 0;                  // most entries of one block
+    int max_read = 0, nread = 0;       // most entries of one block; all
     void* d_whole = nullptr;           // the allocation all of a whole halo's arrays are in
     size_t b_whole = 0;
 };
@@ -250,9 +250,11 @@ struct rbffd_pde {
     int path = 0, launches = 0;  // of the last advance: RBFFD_PATH_*, and its kernel launches
     // Its bounded waits: the status word (host-mapped) a launch that gave up leaves
     // DEV_STATUS_WAIT_TIMEOUT in until the state is set again, whether the next
-    // launches give up, and the time up to which the steps are known to be complete
+    // launches read words nobody publishes (injected), and the time up to which the steps are known to be complete
     int* wait = nullptr;
     int inject_wait = 0;
+    int* inject_rnode = nullptr;
+    size_t inject_bytes = 0;
     double t_sure = 0.0;
     int grid_skip = 0;  // advances left before memory it did not get is asked for again
     int arith = 0;  // RBFFD_ARITH_*

@@ -1534,10 +1534,11 @@ size_t pde_bytes(const rbffd_grid* g, const rbffd_pde_params* prm)
     return b;
 }
 
-// The device-resident RK4's stage inputs with their stage numbers, then its gave-up flag.
+// The device-resident RK4's stage inputs with their stage numbers, those of a node
+// nobody publishes (inject_rnode), then its gave-up flag.
 static size_t word_bytes(const rbffd_pde* P)
 {
-    return 4 * (size_t)P->g->N * P->T * (P->dtype == RBFFD_F64 ? 8 : 4) + 16;
+    return 4 * (size_t)P->g->N * P->T * (P->dtype == RBFFD_F64 ? 8 : 4) + 16 * (size_t)P->T + 16;
 }
 static int* word_gave_up(const rbffd_pde* P) { return (int*)((char*)P->word + word_bytes(P) - 16); }
 
@@ -1583,6 +1584,7 @@ static void pde_free(rbffd_pde* P)
     for (int k = 0; k < 3; k++) dev_free(ctx, P->ws[k], (size_t)P->g->N32 * P->g->n4 * sizeof(float));
     dev_free(ctx, P->comp, (size_t)P->g->N * P->T * sizeof(float));
     dev_free(ctx, P->word, word_bytes(P));
+    dev_free(ctx, P->inject_rnode, P->inject_bytes);
     ctx_wait_release(ctx, P->wait);
     delete P;
 }
@@ -2352,7 +2354,7 @@ static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const Gri
     gp.word[1] = (char*)P->word + 2 * (size_t)g->N * P->T * sizeof(T);
     gp.status = P->wait;  // one address on host and device (unified addressing)
     gp.gave_up = word_gave_up(P);
-    gp.fail = P->inject_wait;
+    if (P->inject_wait) gp.rnode = P->inject_rnode;
     gp.c[0] = gp.c[1] = s0.c;
     gp.c[2] = make_params<T>(P, 2, dt).c;
     gp.c[3] = s3.c;
@@ -2410,6 +2412,19 @@ static int advance_grid(rbffd_pde* P, double dt, int nsteps)
         P->bytes += bytes;
     }
     P->grid_skip = 0;
+    if (P->inject_wait && !P->inject_rnode) {  // every word read is that of node N, which no block owns
+        const std::vector<int> none(std::max(1, q.h->nread), P->g->N);
+        const size_t b = none.size() * sizeof(int);
+        if (dev_alloc(ctx, (void**)&P->inject_rnode, b) != RBFFD_OK) return 0;
+        P->inject_bytes = b;
+        if (cudaMemcpyAsync(P->inject_rnode, none.data(), b, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess) {
+            cudaGetLastError();
+            dev_free(ctx, P->inject_rnode, b);
+            P->inject_rnode = nullptr;
+            return 0;
+        }
+    }
     int done = 0;
     const cudaError_t e = P->dtype == RBFFD_F64 ? advance_grid_t<double>(P, dt, nsteps, q, s, &done)
                                                 : advance_grid_t<float>(P, dt, nsteps, q, s, &done);

@@ -51,7 +51,6 @@ struct GridParams {
     void* word[2];                 // stage inputs with their stage numbers, by parity
     int* status;                   // host-mapped; DEV_STATUS_WAIT_TIMEOUT on a wait that ran out
     int* gave_up;                  // the same for launches that follow, in device memory
-    int fail;                      // nonzero: the first wait counts as run out (injected)
     T c[4];                        // dt/2, dt/2, dt, dt/6
     T kappa;
     int nc, T_tr, R, cs, H, nr, nsteps;  // cs: chunks in shared memory; H: halo positions; nr: most words read
@@ -324,8 +323,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_rk4_grid(GridParams<T> gp)
                 }
         if (!publish) break;
         // the neighbours' values of this stage: one word per thread, or four in flight
-        const int words = nread * TT;
         bool late = false;
+        const int words = nread * TT;
         if (words <= TH) {
             if (tid < words) {
                 const int k = tid / TT, t = tid - k * TT;
@@ -372,7 +371,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_rk4_grid(GridParams<T> gp)
                     }
             }
         }
-        if (late || (gp.fail && words > 0)) s_fail = 1;
+        if (late) s_fail = 1;
         __syncthreads();
         if (s_fail) {
             if (tid == 0) {
