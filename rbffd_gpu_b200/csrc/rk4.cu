@@ -2200,6 +2200,25 @@ struct GridGeom {
 //     (40962, 50, T = 4, three operators); FP32 only with every chunk on chip
 //     (6.4, 5.7 at n = 50; a part: 9.1, 9.6 at n = 101).  More tracers lost
 //     (8.7, 9.6 at 20000, 50, T = 16): too few warps for their gathers.
+// Where it loses within these bounds, and is not taken:
+//   Long rows on small grids, one tracer: a row is one lane's chain here, while the
+//     per-stage kernels split it over up to 16 lanes.  13.8, 36.5 (920, 856, FP64,
+//     three operators), 5.5, 6.7 (1369, 613, FP32 heat), 2.9, 3.1 (1200, 255; but 6.2,
+//     5.5 with three operators in FP64); the
+//     more rows, the less there is to split: 3.45, 3.49 (1845, 277, FP32 heat), 4.1,
+//     3.8 (2470, 318), 13.1, 12.2 (7969, 270, FP64, three operators), but 22.2,
+//     26.7 (5499, 524).
+//   FP64, what a stage reads from L2 beyond it or nearly (as a multiple of the L2):
+//     two operators with two items per thread, whose loads are not issued ahead,
+//     past 0.9: 29.4, 32.0 (163842, 50: 0.98), 28.1, 30.6 (170534, 45: 0.93), but
+//     14.1, 10.9 (163842, 31: 0.53); three operators past 1.055: 35.5, 41.2 (87246,
+//     87: 1.30), 30.2, 33.8 (79349, 80: 1.06), 30.4, 35.0 (64204, 95, T = 2: 1.06),
+//     but 30.9, 28.9 (63943, 99: 1.053).  One operator has no such line: 32.2, 27.5
+//     (163842, 101: 1.04), 33.6, 28.7 (163842, 105: 1.09), 33.0, 34.8 (175266, 100:
+//     1.11), 32.0, 32.8 (155000, 107: 1.03); it is taken.
+//   FP64, three operators, four tracers, less than a sixth on chip: 27.3, 30.4
+//     (50000, 90: 3 of 23 chunks), 21.5, 23.1 (75000, 50: 2 of 13), but 25.0, 20.6
+//     (30000, 120: 6 of 30).
 static bool grid_geom(rbffd_pde* P, GridGeom* out)
 {
     rbffd_ctx* ctx = P->ctx;
@@ -2222,7 +2241,9 @@ static bool grid_geom(rbffd_pde* P, GridGeom* out)
     q.maxt = q.ipt == 2 ? 640 : (items <= 256 ? 256 : (items <= 512 ? 512 : 1024));
     const int nr = std::min(g->nc, grid_reg_chunks(K, es, q.ipt));  // chunks in registers
     const size_t room = (size_t)optin - 256, chunk = (size_t)q.R * (4 * K * es + 8);
-    const int least = (q.vec == 4 ? g->nc : (g->nc + 7) / 8) - nr;            // chunks shared memory has to hold
+    const int part = q.vec == 4 ? 1 : (f64 && K == 3 && P->T == 4 ? 6 : 8);
+    const int least = (g->nc + part - 1) / part - nr;                        // chunks shared memory has to hold
+    if (P->T == 1 && g->n4 > (K == 1 ? 240 : 256) && g->n4 > std::min(480, g->N * 2 / 13)) return false;
     if (least > (int)(room / chunk)) return false;                           // before the halo is built
     int H = 0, words = 0;
     if (grid_halo_whole_sizes(g, q.R, &H, &words) != RBFFD_OK) return false;
@@ -2232,6 +2253,12 @@ static bool grid_geom(rbffd_pde* P, GridGeom* out)
     };
     while (q.cs > 0 && smem(q.cs) > room) q.cs--;
     if (q.cs < least || smem(q.cs) > room) return false;
+    if (f64 && K > 1) {
+        int l2 = 0;
+        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
+        const double past = (double)g->N32 * 4 * (g->nc - nr - q.cs) * (K * es + 2) / std::max(1, l2);
+        if (K == 2 ? q.ipt == 2 && past > 0.9 : past > 1.055) return false;
+    }
     q.smem = smem(q.cs);
     q.threads = round_up((int)((items + q.ipt - 1) / q.ipt), 32);
     if (q.maxt == 256)  // enough threads for the words read, too
