@@ -21,8 +21,14 @@
 // third axis, so a lane looks up one (first, second) pair of coordinates: one
 // run of points on the shell's faces, two single cells inside, and the warp
 // takes the points of all its lanes' runs 32 at a time.  After a shell, n
-// candidates below the searched reach (R times the smallest cell edge) prove
-// that no unvisited point can enter; only those candidates are sorted.
+// candidates below the searched reach prove that no unvisited point can enter;
+// only those candidates are sorted.  The reach is R times the smallest cell edge
+// of the axes along which there are cells left to visit: on a flat or straight
+// point set the thin axes, whose cells are all visited at once, do not hold the
+// search open (40000 points in a plane, n = 31: 136 ms a call while they did, 1.8
+// now).  The runs' places are passed between lanes in registers: in shared memory
+// they cost the ninth block of an SM (1.37, 1.32 ms at 163842 nodes, n = 50; 32.5,
+// 29.9 ms at 40962, 31, half of the points in a thousandth of the box's width).
 //
 // Bound by the sort and the shells' look-ups.  163842 nodes, n = 50: 1.4 ms of
 // kernels, 5.3 ms with one cell looked up at a time by the whole warp and every
@@ -48,7 +54,7 @@ constexpr int KNN_WARPS = 4;        // queries per block
 constexpr int KNN_MAX_N = KNN_CAP / 2 - 1;
 
 struct CellGrid {
-    double lo[3], hc[3], minh;
+    double lo[3], hc[3];
     int dims[3];
 };
 
@@ -217,7 +223,6 @@ k_knn(const double4* __restrict__ pts, const int* __restrict__ start, CellGrid G
     constexpr unsigned FULL = 0xffffffffu;
     __shared__ double sd[KNN_WARPS][KNN_CAP];
     __shared__ int si[KNN_WARPS][KNN_CAP];
-    __shared__ int s_off[KNN_WARPS][32], s_first[KNN_WARPS][32], s_len[KNN_WARPS][32], s_second[KNN_WARPS][32];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int qs = blockIdx.x * KNN_WARPS + w;  // query slot in cell order
     if (qs >= N) return;
@@ -261,25 +266,21 @@ k_knn(const double4* __restrict__ pts, const int* __restrict__ start, CellGrid G
                 if (lane >= o) upto += v;
             }
             const int total = __shfl_sync(FULL, upto, 31);
-            __syncwarp();
-            s_off[w][lane] = upto - len - len2;
-            s_first[w][lane] = first;
-            s_len[w][lane] = len;
-            s_second[w][lane] = second;
-            __syncwarp();
+            const int off = upto - len - len2;
             for (int t = 0; t < total; t += 32) {
                 if (cnt + 32 > KNN_CAP) {  // full: keep the best n + 1
                     warp_bitonic_sort<DESC>(d, id, cnt, lane);
                     cnt = n + 1;
                 }
                 const int e = t + lane;
-                if (e < total) {
-                    int o = 0;  // the last lane whose runs begin at or before e
+                int o = 0;  // the last lane whose runs begin at or before e
 #pragma unroll
-                    for (int h = 16; h > 0; h >>= 1)
-                        if (s_off[w][o + h] <= e) o += h;
-                    const int k = e - s_off[w][o];
-                    const double4 p = pts[k < s_len[w][o] ? s_first[w][o] + k : s_second[w][o] + k - s_len[w][o]];
+                for (int h = 16; h > 0; h >>= 1)
+                    if (__shfl_sync(FULL, off, o + h) <= e) o += h;
+                const int k = e - __shfl_sync(FULL, off, o), l1 = __shfl_sync(FULL, len, o);
+                const int f1 = __shfl_sync(FULL, first, o), f2 = __shfl_sync(FULL, second, o);
+                if (e < total) {
+                    const double4 p = pts[k < l1 ? f1 + k : f2 + k - l1];
                     const double dx = __dsub_rn(q.x, p.x), dy = __dsub_rn(q.y, p.y), dz = __dsub_rn(q.z, p.z);
                     double v = __dmul_rn(dx, dx);
                     v = __dadd_rn(v, __dmul_rn(dy, dy));
@@ -292,11 +293,16 @@ k_knn(const double4* __restrict__ pts, const int* __restrict__ start, CellGrid G
             }
         }
         if (cnt >= n) {
-            const double reach = R * G.minh, r2 = reach * reach;  // every unvisited point is at least reach away
+            // every unvisited point is at least reach away, along an axis with cells left
+            double reach = INFINITY;
+            for (int a = 0; a < 3; a++)
+                if (cc[a] - R > 0 || cc[a] + R < G.dims[a] - 1) reach = fmin(reach, R * G.hc[a]);
+            const bool all = isinf(reach);
+            const double r2 = reach * reach;
             int below = 0;
             for (int t = 0; t < cnt; t += 32)
                 below += __popc(__ballot_sync(FULL, t + lane < cnt && d[t + lane] < r2));
-            if (below < n && R < maxr) continue;
+            if (below < n && !all && R < maxr) continue;
             if (below >= n) {  // the list is among these
                 int kept = 0;
                 for (int t = 0; t < cnt; t += 32) {
@@ -397,7 +403,6 @@ static int stencils_gpu(rbffd_ctx* ctx, const double* xyz, int N, int n, int met
             G.dims[a] = std::max(1, std::min(400, (int)std::ceil((hi[a] - lo[a]) / h) + 1));
             G.hc[a] = std::max((hi[a] - lo[a]) / G.dims[a], 1e-300) * (1.0 + 1e-12);
         }
-        G.minh = std::min(G.hc[0], std::min(G.hc[1], G.hc[2]));
         const size_t ncell = (size_t)G.dims[0] * G.dims[1] * G.dims[2], nstart = ncell + 2;
         const int tiles = (int)((nstart + SCAN_TILE - 1) / SCAN_TILE);
         b_start = (nstart + tiles) * sizeof(int);
