@@ -245,9 +245,13 @@ int rbffd_weights_compute(rbffd_grid* grid, const rbffd_weight_params* params, c
  * A method that does not apply to a system size leaves that size to the
  * autotuner. */
 enum { RBFFD_ELIM_AUTO = 0, RBFFD_ELIM_UNBLOCKED = 1, RBFFD_ELIM_BLOCKED = 2, RBFFD_ELIM_ROW_MAP = 3,
-       RBFFD_ELIM_REGISTERS = 4 };
+       RBFFD_ELIM_REGISTERS = 4,
+       RBFFD_ELIM_ROWS = 5 /* reported only: AUTO's own */ };
 int rbffd_weights_set_elimination(rbffd_ctx* ctx, int method);
 int rbffd_weights_get_elimination(rbffd_ctx* ctx, int* method);
+/* systems[6]: how many systems of the grid's last rbffd_weights_compute each
+ * elimination (RBFFD_ELIM_*) solved. */
+int rbffd_weights_get_solved(const rbffd_grid* grid, int* systems);
 /* The assembled augmented systems [A | B] (m x (m+K), row-major, K = number
  * of selected operators) of the listed stencils, as the weight solver builds
  * them before elimination: RBFFD::getStencilLHS + getStencilMultiRHS

@@ -17,7 +17,7 @@ F32, F64 = 0, 1
 # FP64 arithmetic of the apply and time-stepping kernels (rbffd_ctx_set_arithmetic):
 # fused multiply-adds (default), or rounded products then sums, the reference build's arithmetic
 ARITH_FUSED, ARITH_UNFUSED = 0, 1
-ELIM_AUTO, ELIM_UNBLOCKED, ELIM_BLOCKED, ELIM_ROW_MAP, ELIM_REGISTERS = 0, 1, 2, 3, 4
+ELIM_AUTO, ELIM_UNBLOCKED, ELIM_BLOCKED, ELIM_ROW_MAP, ELIM_REGISTERS, ELIM_ROWS = 0, 1, 2, 3, 4, 5
 X, Y, Z, LAPL, R, HV, LAMBDA, THETA = 0x1, 0x2, 0x4, 0x8, 0x10, 0x20, 0x40, 0x80
 LSFC, XSFC, YSFC, ZSFC, INTERP = 0x100, 0x200, 0x400, 0x800, 0x8000
 ALT_XSFC, ALT_YSFC, ALT_ZSFC = 0x1000, 0x2000, 0x4000
@@ -319,7 +319,7 @@ class Context:
 
     def setWeightsElimination(self, method):
         """Elimination of the batched weight solves on this context: ELIM_AUTO
-        (autotuned per system size), ELIM_UNBLOCKED, ELIM_BLOCKED, ELIM_ROW_MAP
+        (one row per thread, ELIM_ROWS), ELIM_UNBLOCKED, ELIM_BLOCKED, ELIM_ROW_MAP
         or ELIM_REGISTERS; every method gives the same weights bit for bit."""
         self.check(self.L.rbffd_weights_set_elimination(self.h, method), "set_elimination")
 
@@ -465,6 +465,13 @@ class RBFFD:
         ctx.check(ctx.L.rbffd_weights_compute(self.grid.h, ctypes.byref(p), _dp(self.var_epsilon), 0.0,
                                               None if self.deg_per_row is None else _ip(self.deg_per_row)),
                   "rbffd_weights_compute")
+
+    def getSolvedSystems(self):
+        """{ELIM_*: systems} of the last weight solve on this grid (rbffd_weights_get_solved)."""
+        n = (ctypes.c_int * 6)()
+        ctx = self.grid.ctx
+        ctx.check(ctx.L.rbffd_weights_get_solved(self.grid.h, n), "rbffd_weights_get_solved")
+        return {k: v for k, v in enumerate(n) if v}
 
     def setWeights(self, which, w):
         w = _f64(w)

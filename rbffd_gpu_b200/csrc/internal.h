@@ -129,6 +129,7 @@ struct rbffd_grid {
     Kept idx_caller, field[3];
     int wide_applies = 0;
     std::mutex apply_mu;  // one call at a time uses them
+    int solved[6] = {};                 // systems of the last weight solve by elimination (RBFFD_ELIM_*)
     struct WeightsWork* ww = nullptr;   // the weight solver's device workspace and captured launch (weights.cu)
     size_t bytes = 0;
 };

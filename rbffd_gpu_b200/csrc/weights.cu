@@ -1814,6 +1814,8 @@ extern "C" int rbffd_weights_compute(rbffd_grid* g, const rbffd_weight_params* p
         C.rpt = best.rpt;
         if (C.blocked == ELIM_ROWS) C.lda = rows_lda(C.m, K);
     }
+    for (int& n : g->solved) n = 0;
+    for (int c = 0; c < P.nclasses; c++) g->solved[P.cls[c].blocked + 1] += P.cls[c].nrows;  // RBFFD_ELIM_*: one on
     // the whole batch: one persistent launch per class, largest systems first,
     // captured in a CUDA graph and replayed while the parameters stay the same
     WParams Qc[MAX_CLASSES];
@@ -1878,6 +1880,13 @@ extern "C" int rbffd_weights_set_elimination(rbffd_ctx* ctx, int method)
         return set_error(ctx, RBFFD_ERR_INVALID, "unknown elimination %d", method);
     std::lock_guard<std::mutex> lk(ctx->mu);
     ctx->weights_elim = method;
+    return RBFFD_OK;
+}
+
+extern "C" int rbffd_weights_get_solved(const rbffd_grid* g, int* systems)
+{
+    if (!g || !systems) return RBFFD_ERR_INVALID;
+    memcpy(systems, g->solved, sizeof g->solved);
     return RBFFD_OK;
 }
 

@@ -8,3 +8,7 @@ def test_wait_failure():
 
 def test_path():
     assert _lib.load().rbffd_pde_get_path(None, None, None) == -1
+
+
+def test_solved_systems():
+    assert _lib.load().rbffd_weights_get_solved(None, None) == -1
