@@ -1534,13 +1534,13 @@ size_t pde_bytes(const rbffd_grid* g, const rbffd_pde_params* prm)
     return b;
 }
 
-// The device-resident RK4's stage inputs with their stage numbers, those of a node
-// nobody publishes (inject_rnode), then its gave-up flag.
+// The device-resident RK4's gave-up flag (GRID_HEAD bytes), stage inputs with their
+// stage numbers, and those of a node nobody publishes (inject_rnode).
 static size_t word_bytes(const rbffd_pde* P)
 {
-    return 4 * (size_t)P->g->N * P->T * (P->dtype == RBFFD_F64 ? 8 : 4) + 16 * (size_t)P->T + 16;
+    return 4 * (size_t)P->g->N * P->T * (P->dtype == RBFFD_F64 ? 8 : 4) + 16 * (size_t)P->T + GRID_HEAD;
 }
-static int* word_gave_up(const rbffd_pde* P) { return (int*)((char*)P->word + word_bytes(P) - 16); }
+static char* word_first(const rbffd_pde* P) { return (char*)P->word + GRID_HEAD; }
 
 // Whether a device-resident launch that has ended gave up waiting: the state is
 // then a mixture of steps, and the time returns to the last known complete one.
@@ -1816,7 +1816,7 @@ extern "C" int rbffd_pde_set_state(rbffd_pde* P, const double* u)
     }
     RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
     if (pde_gave_up(P)) {  // no launch is left: the new state starts afresh
-        RBFFD_CUDA_TRY(ctx, cudaMemsetAsync(word_gave_up(P), 0, sizeof(int), s));
+        RBFFD_CUDA_TRY(ctx, cudaMemsetAsync(P->word, 0, GRID_HEAD, s));
         RBFFD_CUDA_TRY(ctx, cudaStreamSynchronize(s));
         *(volatile int*)P->wait = DEV_STATUS_OK;
     }
@@ -2377,10 +2377,9 @@ static cudaError_t advance_grid_t(rbffd_pde* P, double dt, int nsteps, const Gri
     gp.cv = s0.cv;
     gp.u = s0.u;
     gp.comp = (float*)P->comp;
-    gp.word[0] = P->word;
-    gp.word[1] = (char*)P->word + 2 * (size_t)g->N * P->T * sizeof(T);
+    gp.word[0] = word_first(P);
+    gp.word[1] = word_first(P) + 2 * (size_t)g->N * P->T * sizeof(T);
     gp.status = P->wait;  // one address on host and device (unified addressing)
-    gp.gave_up = word_gave_up(P);
     if (P->inject_wait) gp.rnode = P->inject_rnode;
     gp.c[0] = gp.c[1] = s0.c;
     gp.c[2] = make_params<T>(P, 2, dt).c;
