@@ -322,7 +322,7 @@ def device_resident(pde):
 
 def stage_kernel_name(shape, tname, resident):
     if resident:
-        return "k_rk4_grid<%s,HEAT> (every step of an advance in one cooperative launch, 16-bit local indices)" % tname
+        return "k_rk4_grid<%s,HEAT> (many steps in each cooperative launch, 16-bit local indices)" % tname
     if shape[2] > 0:
         return "k_stage_tile<%s,HEAT> (halo tile of %d rows, 16-bit local indices)" % (tname, shape[2])
     return "k_stage_scalar<%s,HEAT> (%d lane(s) per row)" % (tname, shape[0])
@@ -996,7 +996,7 @@ def bench_weights(R, torch, ctx):
                              "launch per operator",
         "knn": {"host_s": t_knn, "gpu_s": t_knn_gpu, "gpu_equals_host": knn_equal,
                 "note": "n=101 nearest neighbours of 1e6 nodes; host: exact cell search on all host threads; "
-                        "gpu: rbffd_stencils_knn_gpu including host binning and transfers"},
+                        "gpu: rbffd_stencils_knn_gpu including binning and transfers"},
         "max_abs_derivative_of_constant": worst_const,
         "max_abs_reproduction_error_xyz_degree1_rows": worst_lin,
         "cpu_baseline": {"stencils_per_s": S / cpu_s, "fp64_gflops": cpu_flops / cpu_s / 1e9, "cores": nth,

@@ -131,7 +131,7 @@ int rbffd_variable_epsilon(int N, const double* xyz, int n_pad, const int* st, c
 int rbffd_stencils_generate(const double* xyz, int N, int n, int method, double max_radius, int* st, int* st_len,
                             int* ties, int nthreads);
 /* The same stencils (identical lists and tie count) computed on ctx's device:
- * the host bins the points into a uniform cell grid, one warp per node
+ * the points are binned into a uniform cell grid there too, one warp per node
  * searches the surrounding cells.  Replaces the same reference call
  * (grid_interface.cpp:688-725, KDTree.h:407-433); n <= 255. */
 int rbffd_stencils_knn_gpu(rbffd_ctx* ctx, const double* xyz, int N, int n, int* st, int* ties);
@@ -462,11 +462,12 @@ int rbffd_heat_rk4_noalloc(rbffd_grid* grid, int dtype, double kappa, double dt,
  * RBFFD_ARITH_UNFUSED needs an FP64 one-tracer PDE (else RBFFD_ERR_UNSUPPORTED)
  * and fixes the stage kernel to one lane per row (set_shape may still pick the
  * block size; tiled shapes are refused).  Setting RBFFD_ARITH_FUSED returns the
- * PDE to the autotuned shape. */
+ * PDE to the default (rbffd_pde_advance). */
 int rbffd_pde_set_arithmetic(rbffd_pde* pde, int arith);
 int rbffd_pde_get_arithmetic(rbffd_pde* pde, int* arith);
 /* Kernel-shape choice for this PDE's stage kernel (lanes per stencil row and
- * threads per block); 0 = autotuned. */
+ * threads per block); both 0: the default, device-resident where it applies
+ * (rbffd_pde_advance), else autotuned. */
 int rbffd_pde_set_shape(rbffd_pde* pde, int lanes_per_row, int block_threads);
 int rbffd_pde_get_shape(rbffd_pde* pde, int* lanes_per_row, int* block_threads);
 /* Tiled stage kernel: each thread block takes rows_per_block consecutive rows
@@ -501,8 +502,9 @@ int rbffd_pde_get_shape(rbffd_pde* pde, int* lanes_per_row, int* block_threads);
  * (flags = 1, the former stream_weights argument, keeps its meaning.)
  * Returns RBFFD_ERR_UNSUPPORTED if the staged data do not fit shared memory
  * or the flags do not apply to the PDE.
- * get_tiling reports 0 when the stage kernel gathers from global memory;
- * get_tile_flags the flags of the shape in use (set or autotuned). */
+ * get_tiling reports 0 when the stage kernel gathers from global memory or the
+ * steps ran device-resident; get_tile_flags the flags of the shape in use (set or
+ * autotuned), 0 in the same cases. */
 enum {
     RBFFD_TILE_STREAM_WEIGHTS = 1,
     RBFFD_TILE_SLOT_SCHEDULE = 2,

@@ -662,7 +662,7 @@ class TimeDependentPDE:
 
     def setArithmetic(self, arith):
         """ARITH_UNFUSED (FP64, one tracer): the reference build's arithmetic,
-        one lane per stencil row; ARITH_FUSED: fused multiply-adds, autotuned shape."""
+        one lane per stencil row; ARITH_FUSED: fused multiply-adds, the default path."""
         self.ctx.check(self.ctx.L.rbffd_pde_set_arithmetic(self.h, arith), "set_arithmetic")
 
     def getArithmetic(self):

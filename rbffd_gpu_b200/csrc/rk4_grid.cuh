@@ -26,10 +26,12 @@
 // One lane per (row, tracer), slots in stencil order: the arithmetic of
 // k_stage_scalar and k_stage_vec with one lane per row, bit for bit.
 //
-// What bounds it: on small grids the exchange, about 1 us (a store to L2 and one
-// or two polls of it), then a row's chain of gathers and multiply-adds; on large
-// ones the shared-memory gathers, and the L2 reads of what does not fit.  The
-// times at which the per-stage kernels lose to it are at grid_geom (rk4.cu).
+// What bounds it, in cycles of a stage read with clock64 (a busy warp's): a row's
+// chain of gathers and multiply-adds with the update, then the exchange (a store to
+// L2, polls until it is seen, a barrier).  642 nodes (n = 17, FP64): 820 and 1410;
+// 4096 (31, three operators): 1340 and 1080 to 1280; 40003 (37, FP32): 2010 and 1290
+// to 1400; 163842 (50, FP64), with the L2 reads of what does not fit: 17000 and 1700
+// to 2000.  Where the per-stage kernels are faster is at grid_geom (rk4.cu).
 #pragma once
 
 constexpr int GRID_POLL_LIMIT = 1 << 21;  // polls of one word (about a second)

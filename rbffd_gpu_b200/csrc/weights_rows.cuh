@@ -441,7 +441,8 @@ __device__ void rows_back_substitute_t(const double* a, double* scratch, int m, 
     }
 }
 
-// KB right-hand sides at once per warp: as many as leave no warp with a second round, up to 4.
+// KB right-hand sides at once per warp: as many as leave no warp with a second
+// round, up to 3; a warp with more takes further rounds (8 operators on one warp: three).
 template <int NW, int BS, typename OutF>
 __device__ void rows_back_substitute(const double* a, double* scratch, int m, int K, int lda, OutF out)
 {
