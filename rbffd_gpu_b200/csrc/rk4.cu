@@ -2332,13 +2332,19 @@ static cudaError_t grid_ordered(rbffd_ctx* ctx, int blocks, const std::function<
     }
     std::vector<rbffd_ctx*> busy;  // the others' unfinished launches
     int total = blocks;
-    for (rbffd_ctx* c : L->ctxs) {
-        if (c->grid_blocks > 0 && cudaEventQuery(c->grid_event) == cudaSuccess) c->grid_blocks = 0;
-        if (c == ctx || c->grid_blocks == 0) continue;
-        busy.push_back(c);
-        total += c->grid_blocks;
+    if (L->ctxs.size() > 1) {
+        // a query would break a capture that another thread makes in the global mode
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        for (rbffd_ctx* c : L->ctxs) {
+            if (c->grid_blocks > 0 && cudaEventQuery(c->grid_event) == cudaSuccess) c->grid_blocks = 0;
+            if (c == ctx || c->grid_blocks == 0) continue;
+            busy.push_back(c);
+            total += c->grid_blocks;
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        cudaGetLastError();  // cudaErrorNotReady
     }
-    cudaGetLastError();  // cudaErrorNotReady
     std::sort(busy.begin(), busy.end(), [](const rbffd_ctx* a, const rbffd_ctx* b) { return a->grid_blocks > b->grid_blocks; });
     for (size_t k = 0; k < busy.size() && total > ctx->sm_count; k++) {
         e = cudaStreamWaitEvent(ctx->stream, busy[k]->grid_event, 0);

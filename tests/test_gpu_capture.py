@@ -46,3 +46,45 @@ def test_replayed_advance(T, advance_first, graph):
     ref.close()
     grid.close()
     c.close()
+
+
+def test_advance_beside_another_capture():
+    """An asynchronous advance of a context that shares the device with another,
+    issued while a thread captures a stream of its own in the global mode."""
+    N, n = 3000, 31
+    xyz, st = sphere_problem(N, n, 3)
+    runs = []
+    for k in range(2):
+        c = R.Context(0)
+        grid = R.Grid(c, xyz, st)
+        der = R.RBFFD(R.LSFC, grid, 2)
+        der.setWeights(R.LSFC, np.random.default_rng(1).standard_normal((N, n)))
+        pde = R.HeatSphere(grid, der, 0.7, dtype=R.F64)
+        pde.fillInitialConditions(np.random.default_rng(2).standard_normal(N))
+        pde.advance(R.RK4, 1e-4, 5)
+        runs.append((c, grid, der, pde))
+    x = torch.ones(1000, device="cuda")
+    torch.cuda.synchronize()
+    recorded = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(recorded):
+        y = x + 1
+        for c, grid, der, pde in runs:  # another stream, which is not captured
+            pde.advance(R.RK4, 1e-4, 20, asynchronous=True)
+        y = y * 2
+    recorded.replay()
+    torch.cuda.synchronize()
+    assert float(y.sum()) == 4000.0
+    out = [pde.getLocalSolution() for c, grid, der, pde in runs]
+    assert np.array_equal(*out)
+    c, grid, der, pde = runs[0]
+    ref = R.HeatSphere(grid, der, 0.7, dtype=R.F64)
+    ref.setShape(1, 128)
+    ref.fillInitialConditions(np.random.default_rng(2).standard_normal(N))
+    ref.advance(R.RK4, 1e-4, 25)
+    assert np.array_equal(out[0], ref.getLocalSolution())
+    ref.close()
+    recorded.reset()
+    for c, grid, der, pde in runs:
+        pde.close()
+        grid.close()
+        c.close()
